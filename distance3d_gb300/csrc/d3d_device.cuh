@@ -51,6 +51,68 @@ __device__ __forceinline__ float sqrt_t(float a) { return sqrtf(a); }
 __device__ __forceinline__ double abs_t(double a) { return fabs(a); }
 __device__ __forceinline__ float abs_t(float a) { return fabsf(a); }
 
+// Comparisons: x < y, x <= y, x > 0, x < 0, x >= 0, x <= 0, false for a NaN
+// operand.  A double compare runs on the FP64 pipe like any FP64 instruction
+// (one warp instruction per 16 cycles of the SM, 110 cycles of latency), while
+// the integer pipe is idle in the FP64 kernels: a compare of the bit patterns
+// measured 11 cycles per sub-partition and 21 of latency.  A unit that lets
+// the compiler contract products (-fmad=true) defines D3D_FP_COMPARES before
+// it includes this file: which of two products is fused depends on the
+// surrounding code, and its results are to stay as they are.
+template <typename T>
+struct Compare {
+    static __device__ __forceinline__ bool lt(T a, T b) { return a < b; }
+    static __device__ __forceinline__ bool le(T a, T b) { return a <= b; }
+    static __device__ __forceinline__ bool above0(T x) { return x > T(0); }
+    static __device__ __forceinline__ bool below0(T x) { return x < T(0); }
+    static __device__ __forceinline__ bool not_below0(T x) { return x >= T(0); }
+    static __device__ __forceinline__ bool not_above0(T x) { return x <= T(0); }
+};
+#ifndef D3D_FP_COMPARES
+template <>
+struct Compare<double> {
+    static constexpr long long kInf = 0x7ff0000000000000ll;
+    // an integer of the same order: -0 equal to +0, the NaNs beyond the infinities
+    static __device__ __forceinline__ long long order(double x) {
+        const long long b = __double_as_longlong(x);
+        return b < 0 ? (long long)(0x8000000000000000ull - (unsigned long long)b) : b;
+    }
+    static __device__ __forceinline__ unsigned long long bits(double x) {
+        return (unsigned long long)__double_as_longlong(x);
+    }
+    static __device__ __forceinline__ bool lt(double a, double b) {
+        const long long x = order(a), y = order(b);
+        return x < y && x >= -kInf && y <= kInf;
+    }
+    static __device__ __forceinline__ bool le(double a, double b) {
+        const long long x = order(a), y = order(b);
+        return x <= y && x >= -kInf && y <= kInf;
+    }
+    static __device__ __forceinline__ bool above0(double x) { return bits(x) - 1ull < (unsigned long long)kInf; }
+    static __device__ __forceinline__ bool below0(double x) {
+        return bits(x) - 0x8000000000000001ull < (unsigned long long)kInf;
+    }
+    static __device__ __forceinline__ bool not_below0(double x) {
+        return bits(x) <= (unsigned long long)kInf || bits(x) == 0x8000000000000000ull;
+    }
+    static __device__ __forceinline__ bool not_above0(double x) {
+        return bits(x) - 0x8000000000000000ull <= (unsigned long long)kInf || bits(x) == 0ull;
+    }
+};
+#endif
+template <typename T>
+__device__ __forceinline__ bool lt(T a, T b) { return Compare<T>::lt(a, b); }
+template <typename T>
+__device__ __forceinline__ bool le(T a, T b) { return Compare<T>::le(a, b); }
+template <typename T>
+__device__ __forceinline__ bool above0(T x) { return Compare<T>::above0(x); }
+template <typename T>
+__device__ __forceinline__ bool below0(T x) { return Compare<T>::below0(x); }
+template <typename T>
+__device__ __forceinline__ bool not_below0(T x) { return Compare<T>::not_below0(x); }
+template <typename T>
+__device__ __forceinline__ bool not_above0(T x) { return Compare<T>::not_above0(x); }
+
 // np.dot of two 3-vectors (ddot), np.linalg.norm, and the small GEMMs of
 // geometry.py:157 / containment.py:147: fma(a2,b2, fma(a1,b1, a0*b0))
 template <typename T>
@@ -212,9 +274,9 @@ __device__ __forceinline__ int hull_argmax(const T* verts, int off, int nv, V3<T
 // absolute term that covers denormal operands).  A first FP32 pass finds
 // L = max_k (s_k - E_k), a lower bound on the FP64 maximum; the second pass
 // computes the FP64 product only where s_k + E_k >= L, in index order with
-// the strict comparison of hull_argmax.  Every vertex it skips has an FP64
-// product below L, so the index is hull_argmax's, bit for bit.  With a
-// non-finite FP32 value (NaN or infinite coordinates, or magnitudes beyond
+// the strict comparison of hull_argmax, and is left out where one vertex alone
+// reaches L (nearly always).  Every vertex it skips has an FP64 product below
+// L, so the index is hull_argmax's, bit for bit.  With a non-finite FP32 value (NaN or infinite coordinates, or magnitudes beyond
 // FP32) the plain FP64 scan runs instead.
 struct Filter32 {
     float dx, dy, dz, dabs;
@@ -239,17 +301,28 @@ __device__ __forceinline__ float2 filter_product(const float* v32, int row, cons
 __device__ __forceinline__ int hull_argmax_filtered(const double* v64, const float* v32, int off, int nv, V3<double> d) {
     if (nv <= 1) return 0;
     const Filter32 f = filter32(d);
-    float lo = -INFINITY;
+    float lo = -INFINITY, top = -INFINITY, second = -INFINITY;
+    int best = 0;
     bool finite = isfinite(f.dabs);
 #pragma unroll 1
     for (int k = 0; k < nv; ++k) {
         const float2 se = filter_product(v32, off + k, f);
         finite &= isfinite(se.x) && isfinite(se.y);
         lo = fmaxf(lo, se.x - se.y);
+        const float up = se.x + se.y;
+        if (up > top) {
+            second = top;
+            top = up;
+            best = k;
+        } else {
+            second = fmaxf(second, up);
+        }
     }
+    // one vertex alone reaches the bound: it is the maximum, whatever its FP64 product
+    if (finite && second < lo) return best;
     // not finite: every vertex is a candidate, which is hull_argmax's scan
     const bool all = !finite;
-    int best = -1;
+    best = -1;
     double bd = 0.0;
 #pragma unroll 1
     for (int k = 0; k < nv; ++k) {
@@ -257,7 +330,7 @@ __device__ __forceinline__ int hull_argmax_filtered(const double* v64, const flo
         if (all || se.x + se.y >= lo) {
             const V3<double> w = load_vertex(v64, off + k);
             const double x = dot102(w.x, w.y, w.z, d.x, d.y, d.z);
-            if (best < 0 || x > bd) {
+            if (best < 0 || lt(bd, x)) {
                 bd = x;
                 best = k;
             }

@@ -35,6 +35,7 @@
 //
 // Status codes are those of the FP64 EPA.  Compiled with -fmad=true; the
 // tests bound the depth error against the FP64 oracle.
+#define D3D_FP_COMPARES  // see d3d_device.cuh
 #include "capi_util.h"
 #include "epa_mixed.h"
 #include "epa_mixed.cuh"

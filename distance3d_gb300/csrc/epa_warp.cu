@@ -36,6 +36,7 @@
 // behind a pinched horizon are FP32 noise on nearly coplanar faces, which
 // FP64 resolves.  Its own fallback pairs go to the serial FP64 EPA (the
 // reference's arithmetic).  Compiled with -fmad=true.
+#define D3D_FP_COMPARES  // see d3d_device.cuh
 #include "capi_util.h"
 #include "epa_mixed.cuh"
 #include "epa_mixed.h"

@@ -43,6 +43,7 @@
 // rows plus the gap row, against ~17-19 FP64 iterations for the plain form.
 // Compiled with -fmad=true: the tests bound its error against the FP64
 // oracle.
+#define D3D_FP_COMPARES  // see d3d_device.cuh
 #include <cub/cub.cuh>
 
 #include "capi_util.h"

@@ -44,8 +44,8 @@ template <typename T>
 __device__ __forceinline__ void bary_line(V3<T> a, V3<T> b, const JoltEps<T>& E, T& u, T& v) {
     V3<T> ab = b - a;
     T den = dot(ab, ab);
-    if (den < E.sq) {
-        if (dot(a, a) < dot(b, b)) {
+    if (lt(den, E.sq)) {
+        if (lt(dot(a, a), dot(b, b))) {
             u = T(1);
             v = T(0);
         } else {
@@ -67,11 +67,11 @@ template <typename T, bool SCALED = false>
 __device__ __forceinline__ void bary_plane(V3<T> a, V3<T> b, V3<T> c, const JoltEps<T>& E, T& u, T& v, T& w) {
     V3<T> v0 = b - a, v1 = c - a, v2 = c - b;
     T d00 = dot(v0, v0), d11 = dot(v1, v1), d22 = dot(v2, v2);
-    if (d00 <= d22) {
+    if (le(d00, d22)) {
         T d01 = dot(v0, v1);
         T den = d00 * d11 - d01 * d01;
-        if (abs_t(den) < (SCALED ? E.plane * (d00 * d11) : E.plane)) {
-            if (d00 > d11) {
+        if (lt(abs_t(den), SCALED ? E.plane * (d00 * d11) : E.plane)) {
+            if (lt(d11, d00)) {
                 bary_line(a, b, E, u, v);
                 w = T(0);
             } else {
@@ -87,8 +87,8 @@ __device__ __forceinline__ void bary_plane(V3<T> a, V3<T> b, V3<T> c, const Jolt
     } else {
         T d12 = dot(v1, v2);
         T den = d11 * d22 - d12 * d12;
-        if (abs_t(den) < (SCALED ? E.plane * (d11 * d22) : E.plane)) {
-            if (d11 > d22) {
+        if (lt(abs_t(den), SCALED ? E.plane * (d11 * d22) : E.plane)) {
+            if (lt(d22, d11)) {
                 bary_line(a, c, E, u, w);
                 v = T(0);
             } else {
@@ -128,11 +128,11 @@ template <typename T>
 __device__ __forceinline__ V3<T> cp_line(V3<T> a, V3<T> b, const JoltEps<T>& E, int& set) {
     T u, v;
     bary_line(a, b, E, u, v);
-    if (v <= T(0)) {
+    if (not_above0(v)) {
         set = 1;
         return a;
     }
-    if (u <= T(0)) {
+    if (not_above0(u)) {
         set = 2;
         return b;
     }
@@ -145,22 +145,22 @@ __device__ __forceinline__ V3<T> cp_line(V3<T> a, V3<T> b, const JoltEps<T>& E, 
 template <typename T, bool FAST = false>
 __device__ __forceinline__ V3<T> cp_triangle(V3<T> a, V3<T> b, V3<T> c, const JoltEps<T>& E, int& set) {
     V3<T> ab = b - a, ac = c - a, bc = c - b;
-    V3<T> n = (dot(bc, bc) < dot(ac, ac)) ? cross(ab, bc) : cross(ab, ac);
+    V3<T> n = lt(dot(bc, bc), dot(ac, ac)) ? cross(ab, bc) : cross(ab, ac);
     T nl = dot(n, n);
-    if (nl < E.sq) {
+    if (lt(nl, E.sq)) {
         int s, ns;
         V3<T> cp = cp_line(a, b, E, s);
         T best = dot(cp, cp);
         V3<T> q = cp_line(a, c, E, ns);
         T d2 = dot(q, q);
-        if (d2 < best) {
+        if (lt(d2, best)) {
             cp = q;
             best = d2;
             s = (ns & 1) + ((ns & 2) << 1);
         }
         q = cp_line(b, c, E, ns);
         d2 = dot(q, q);
-        if (d2 < best) {
+        if (lt(d2, best)) {
             cp = q;
             s = ns << 1;
         }
@@ -169,37 +169,37 @@ __device__ __forceinline__ V3<T> cp_triangle(V3<T> a, V3<T> b, V3<T> c, const Jo
     }
     V3<T> ap = -a;
     T d1 = dot(ab, ap), d2 = dot(ac, ap);
-    if (d1 <= T(0) && d2 <= T(0)) {
+    if (not_above0(d1) && not_above0(d2)) {
         set = 1;
         return a;
     }
     V3<T> bp = -b;
     T d3 = dot(ab, bp), d4 = dot(ac, bp);
-    if (d3 >= T(0) && d4 <= d3) {
+    if (not_below0(d3) && le(d4, d3)) {
         set = 2;
         return b;
     }
     T vc = d1 * d4 - d3 * d2;
-    if (vc <= T(0) && T(0) <= d1 && d3 <= T(0)) {
+    if (not_above0(vc) && not_below0(d1) && not_above0(d3)) {
         T v = d1 / (d1 - d3);
         set = 3;
         return a + ab * v;
     }
     V3<T> cpp = -c;
     T d5 = dot(ab, cpp), d6 = dot(ac, cpp);
-    if (d6 >= T(0) && d5 <= d6) {
+    if (not_below0(d6) && le(d5, d6)) {
         set = 4;
         return c;
     }
     T vb = d5 * d2 - d1 * d6;
-    if (vb <= T(0) && T(0) <= d2 && d6 <= T(0)) {
+    if (not_above0(vb) && not_below0(d2) && not_above0(d6)) {
         T w = d2 / (d2 - d6);
         set = 5;
         return a + ac * w;
     }
     T va = d3 * d6 - d5 * d4;
     T d43 = d4 - d3, d56 = d5 - d6;
-    if (va <= T(0) && T(0) <= d43 && d56 >= T(0)) {
+    if (not_above0(va) && not_below0(d43) && not_below0(d56)) {
         T w = d43 / (d43 + d56);
         set = 6;
         return b + bc * w;
@@ -222,10 +222,10 @@ __device__ __forceinline__ int outside_planes(V3<T> a, V3<T> b, V3<T> c, V3<T> d
     V3<T> abac = cross(ab, ac), acad = cross(ac, ad), adab = cross(ad, ab), bdbc = cross(bd, bc);
     T sp0 = dot(a, abac), sp1 = dot(a, acad), sp2 = dot(a, adab), sp3 = dot(b, bdbc);
     T sd0 = dot(ad, abac), sd1 = dot(ab, acad), sd2 = dot(ac, adab), sd3 = -dot(ab, bdbc);
-    if (sd0 > T(0) && sd1 > T(0) && sd2 > T(0) && sd3 > T(0))
-        return (sp0 >= -E.plane) | ((sp1 >= -E.plane) << 1) | ((sp2 >= -E.plane) << 2) | ((sp3 >= -E.plane) << 3);
-    if (sd0 < T(0) && sd1 < T(0) && sd2 < T(0) && sd3 < T(0))
-        return (sp0 <= E.plane) | ((sp1 <= E.plane) << 1) | ((sp2 <= E.plane) << 2) | ((sp3 <= E.plane) << 3);
+    if (above0(sd0) && above0(sd1) && above0(sd2) && above0(sd3))
+        return le(-E.plane, sp0) | (le(-E.plane, sp1) << 1) | (le(-E.plane, sp2) << 2) | (le(-E.plane, sp3) << 3);
+    if (below0(sd0) && below0(sd1) && below0(sd2) && below0(sd3))
+        return le(sp0, E.plane) | (le(sp1, E.plane) << 1) | (le(sp2, E.plane) << 2) | (le(sp3, E.plane) << 3);
     return 15;
 }
 
@@ -365,7 +365,7 @@ __device__ __forceinline__ bool closest_to_origin(const Simplex<T, Rows>& S, T p
             int ns;
             const V3<T> q = cp_triangle<T, FAST>(row_of(S.Y, i0), row_of(S.Y, i1), row_of(S.Y, i2), E, ns);
             const T d2 = dot(q, q);
-            if (f == 0 || d2 < best) {
+            if (f == 0 || lt(d2, best)) {
                 best = d2;
                 r = q;
                 s = ((ns & 1) << i0) | (((ns >> 1) & 1) << i1) | (((ns >> 2) & 1) << i2);
@@ -373,7 +373,7 @@ __device__ __forceinline__ bool closest_to_origin(const Simplex<T, Rows>& S, T p
         }
     }
     T l = dot(r, r);
-    if (l < prev) {
+    if (lt(l, prev)) {
         v = r;
         vl = l;
         set = s;
@@ -390,7 +390,7 @@ __device__ __forceinline__ T max_y_len_sq(const Simplex<T, Rows>& S) {
     for (int i = 1; i < 4; ++i)
         if (i < S.n) {
             T l = dot(S.Y[i], S.Y[i]);
-            if (l > m) m = l;
+            if (lt(m, l)) m = l;
         }
     return m;
 }
@@ -539,7 +539,7 @@ __device__ __forceinline__ bool gjk_step_begin(GjkLoop<T, Rows>& g, const d3d_st
     __syncwarp(together);
     V3<T> w = p - q;
     T dd = dot(g.dir, w);
-    if (dd < T(0) && dd * dd > g.vl * max_d2) {
+    if (below0(dd) && lt(g.vl * max_d2, dd * dd)) {
         g.state = GJK_CLIPPED;
         return true;
     }
@@ -574,13 +574,13 @@ __device__ __forceinline__ bool gjk_step_end(GjkLoop<T, Rows>& g, T tol_sq, cons
         return true;
     }
     simplex_compact<T, true>(g.S, set);
-    if (g.vl <= tol_sq || g.vl <= E.isect * max_y_len_sq(g.S)) {
+    if (le(g.vl, tol_sq) || le(g.vl, E.isect * max_y_len_sq(g.S))) {
         g.vl = T(0);
         g.state = GJK_INTERSECTION;
         return true;
     }
     g.dir = -g.dir;
-    if (g.prev - g.vl <= E.conv * g.prev) {
+    if (le(g.prev - g.vl, E.conv * g.prev)) {
         g.state = GJK_NO_INTERSECTION;
         return true;
     }

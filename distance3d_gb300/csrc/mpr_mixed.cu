@@ -16,6 +16,7 @@
 // portal expansions); the collinear test of the portal discovery adds the
 // FP32 noise of |v0 x v1|^2 to the reference's EPSILON so that the
 // origin-on-segment case is found as in FP64.  Compiled with -fmad=true.
+#define D3D_FP_COMPARES  // see d3d_device.cuh
 #include "capi_util.h"
 #include "gjk_mixed.cuh"
 #include "mpr.cuh"
