@@ -1,7 +1,8 @@
 // bvh.cu -- broad phase: a linear BVH over FP64 axis-aligned boxes.
 //
 // Build (all on the device):
-//   1. bounds of the box centers (block reduction + one-block reduction);
+//   1. bounds of the box centers (warp reductions on order-preserving keys,
+//      one atomic per block and bound);
 //   2. 63-bit Morton codes of the centers (21 bits per axis), radix-sorted
 //      with the leaf index as payload (CUB);
 //   3. Karras' (2012) parallel hierarchy: one thread per internal node finds
@@ -9,6 +10,11 @@
 //      by index;
 //   4. bottom-up refit with one atomic visit counter per internal node (no
 //      waiting: the second child to arrive merges and climbs on).
+// A node is one 64-byte record: the boxes of its two children, their ids and
+// the ends of their ranges, so that a traversal step waits for one load.
+// (With child ids, ranges and boxes in arrays of their own a step took three
+// dependent loads: self pairs of a 131,072-collider scene 109 -> 61 us, the
+// 30,011 queries of a 200,003-leaf tree 146 -> 73 us.)
 // Internal node boxes are FP32 rounded outward (lower bounds down, upper
 // bounds up), so a box that overlaps in FP64 also overlaps in FP32: pruning
 // never loses a pair.  Leaves are tested with the caller's exact FP64 boxes
@@ -22,32 +28,37 @@
 #include <cub/cub.cuh>
 
 #include "capi_util.h"
+#include "d3d_device.cuh"
 #include "scratch.h"
 
 namespace {
 
 constexpr int kBlock = 256;
 constexpr int kStack = 128;
-constexpr int kBoundBlocks = 512;
+constexpr uint32_t kRoot = 0xffffffffu;
 
 inline size_t up(size_t x) { return (x + 255) & ~size_t(255); }
 
 // ----------------------------------------------------------- tree layout
 // All arrays live in one caller-provided buffer; offsets depend on n only.
+struct Node {
+    // children 0 and 1: box lower corner (xyz) and id (w, int bits: >= 0 an internal node, ~index of a
+    // leaf), box upper corner (xyz) and last sorted position under the child (w, int bits)
+    float4 child[4];
+};
 struct Tree {
     int64_t n;
+    // one block cleared before a build: error flags (4 int32), then the bounds of the centers as
+    // keys (uint64: largest ~key per axis, largest key per axis)
+    int32_t* flags;
+    unsigned long long* bounds;
     int32_t* sorted;    // [n]   sorted position -> original index
-    int2* child;        // [n-1] children: c >= 0 internal node, c < 0 leaf ~c (sorted position)
-    int2* range;        // [n-1] first/last sorted position under the node
-    float4* box;        // [2(n-1)] internal boxes: lo (xyz), hi (xyz), FP32 outward
-    float4* leafbox;    // [2n]  leaf boxes in sorted order, FP32 outward
-    int32_t* parent;    // [n-1 + n] parents of internal nodes, then of leaves
-    int32_t* visits;    // [n-1] refit counters
+    Node* node;         // [n-1]
+    uint32_t* parent;   // [n-1 + n] parent << 1 | side of internal nodes, then of leaves (kRoot: the root)
+    int32_t* visits;    // [n-1] refit counters, zero between refits
     uint64_t* keys;     // [n]
     uint64_t* keys_out; // [n]
     int32_t* vals;      // [n]
-    double* bounds;     // [2 * 3 * kBoundBlocks + 6]
-    int32_t* flags;     // [4] error flags
     void* cub_temp;
     size_t cub_bytes;
 };
@@ -68,34 +79,27 @@ size_t layout(void* base, int64_t n, Tree* t) {
         off += up(bytes);
         return o;
     };
+    size_t o_flags = take(256);
     size_t o_sorted = take(sizeof(int32_t) * n);
-    size_t o_child = take(sizeof(int2) * ni);
-    size_t o_range = take(sizeof(int2) * ni);
-    size_t o_box = take(sizeof(float4) * 2 * ni);
-    size_t o_leafbox = take(sizeof(float4) * 2 * n);
-    size_t o_parent = take(sizeof(int32_t) * (ni + n));
+    size_t o_node = take(sizeof(Node) * ni);
+    size_t o_parent = take(sizeof(uint32_t) * (ni + n));
     size_t o_visits = take(sizeof(int32_t) * ni);
     size_t o_keys = take(sizeof(uint64_t) * n);
     size_t o_keys_out = take(sizeof(uint64_t) * n);
     size_t o_vals = take(sizeof(int32_t) * n);
-    size_t o_bounds = take(sizeof(double) * (6 * kBoundBlocks + 6));
-    size_t o_flags = take(sizeof(int32_t) * 4);
     size_t o_cub = take(cub_bytes);
     if (t) {
         char* b = static_cast<char*>(base);
         t->n = n;
+        t->flags = reinterpret_cast<int32_t*>(b + o_flags);
+        t->bounds = reinterpret_cast<unsigned long long*>(b + o_flags + 16);
         t->sorted = reinterpret_cast<int32_t*>(b + o_sorted);
-        t->child = reinterpret_cast<int2*>(b + o_child);
-        t->range = reinterpret_cast<int2*>(b + o_range);
-        t->box = reinterpret_cast<float4*>(b + o_box);
-        t->leafbox = reinterpret_cast<float4*>(b + o_leafbox);
-        t->parent = reinterpret_cast<int32_t*>(b + o_parent);
+        t->node = reinterpret_cast<Node*>(b + o_node);
+        t->parent = reinterpret_cast<uint32_t*>(b + o_parent);
         t->visits = reinterpret_cast<int32_t*>(b + o_visits);
         t->keys = reinterpret_cast<uint64_t*>(b + o_keys);
         t->keys_out = reinterpret_cast<uint64_t*>(b + o_keys_out);
         t->vals = reinterpret_cast<int32_t*>(b + o_vals);
-        t->bounds = reinterpret_cast<double*>(b + o_bounds);
-        t->flags = reinterpret_cast<int32_t*>(b + o_flags);
         t->cub_temp = b + o_cub;
         t->cub_bytes = cub_bytes;
     }
@@ -112,45 +116,49 @@ __device__ __forceinline__ void load_box(const double* aabbs, int64_t i, double*
     }
 }
 
-__global__ void k_center_bounds(const double* __restrict__ aabbs, int64_t n, double* __restrict__ partial) {
-    __shared__ double s[6][kBlock];
-    double m[6] = {DBL_MAX, DBL_MAX, DBL_MAX, -DBL_MAX, -DBL_MAX, -DBL_MAX};
+// Unsigned order equals the order of the doubles (not NaN); 0 is below every key.
+__device__ __forceinline__ unsigned long long order_key(double x) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+    return (u >> 63) ? ~u : (u | 0x8000000000000000ull);
+}
+__device__ __forceinline__ double from_key(unsigned long long k) {
+    return __longlong_as_double((long long)((k >> 63) ? (k & 0x7fffffffffffffffull) : ~k));
+}
+
+// The warp's largest 64-bit value, by REDUX on the halves.
+__device__ __forceinline__ unsigned long long warp_max64(unsigned long long k) {
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(k >> 32));
+    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(k >> 32) == hi ? (unsigned)k : 0u);
+    return ((unsigned long long)hi << 32) | lo;
+}
+
+// bounds[k]: largest ~key of the centers on axis k (their minimum), bounds[3 + k]: largest key; NaN
+// centers are left out.  (Partial bounds per block, reduced by one thread, took 178 us at any size: FP64
+// compares one after the other on one lane.)
+__global__ void k_center_bounds(const double* __restrict__ aabbs, int64_t n, unsigned long long* __restrict__ bounds) {
+    unsigned long long m[6] = {};
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double lo[3], hi[3];
         load_box(aabbs, i, lo, hi);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            double c = 0.5 * (lo[k] + hi[k]);
-            m[k] = fmin(m[k], c);
-            m[3 + k] = fmax(m[3 + k], c);
+            const double c = 0.5 * (lo[k] + hi[k]);
+            const unsigned long long key = order_key(c);
+            if (c != c) continue;
+            if (~key > m[k]) m[k] = ~key;
+            if (key > m[3 + k]) m[3 + k] = key;
         }
     }
-#pragma unroll
-    for (int k = 0; k < 6; ++k) s[k][threadIdx.x] = m[k];
+    __shared__ unsigned long long best[6];
+    if (threadIdx.x < 6) best[threadIdx.x] = 0ull;
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) {
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                s[k][threadIdx.x] = fmin(s[k][threadIdx.x], s[k][threadIdx.x + w]);
-                s[3 + k][threadIdx.x] = fmax(s[3 + k][threadIdx.x], s[3 + k][threadIdx.x + w]);
-            }
-        }
-        __syncthreads();
+    for (int k = 0; k < 6; ++k) {
+        const unsigned long long w = warp_max64(m[k]);
+        if ((threadIdx.x & 31) == 0) atomicMax(best + k, w);
     }
-    if (threadIdx.x == 0)
-        for (int k = 0; k < 6; ++k) partial[6 * blockIdx.x + k] = s[k][0];
-}
-
-__global__ void k_reduce_bounds(double* __restrict__ partial, int blocks, double* __restrict__ out) {
-    if (threadIdx.x != 0) return;
-    double m[6] = {DBL_MAX, DBL_MAX, DBL_MAX, -DBL_MAX, -DBL_MAX, -DBL_MAX};
-    for (int b = 0; b < blocks; ++b)
-        for (int k = 0; k < 3; ++k) {
-            m[k] = fmin(m[k], partial[6 * b + k]);
-            m[3 + k] = fmax(m[3 + k], partial[6 * b + 3 + k]);
-        }
-    for (int k = 0; k < 6; ++k) out[k] = m[k];
+    __syncthreads();
+    if (threadIdx.x < 6) atomicMax(bounds + threadIdx.x, best[threadIdx.x]);
 }
 
 __device__ __forceinline__ uint64_t spread21(uint64_t v) {
@@ -163,7 +171,8 @@ __device__ __forceinline__ uint64_t spread21(uint64_t v) {
     return v;
 }
 
-__global__ void k_morton(const double* __restrict__ aabbs, int64_t n, const double* __restrict__ bounds,
+// The scaling is FP32 (after an FP64 subtraction): the codes only shape the tree.
+__global__ void k_morton(const double* __restrict__ aabbs, int64_t n, const unsigned long long* __restrict__ bounds,
                          uint64_t* __restrict__ keys, int32_t* __restrict__ vals) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -172,24 +181,13 @@ __global__ void k_morton(const double* __restrict__ aabbs, int64_t n, const doub
     uint64_t q[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        double ext = bounds[3 + k] - bounds[k];
-        double u = ext > 0.0 ? (0.5 * (lo[k] + hi[k]) - bounds[k]) / ext : 0.0;
-        double x = u * 2097152.0;
-        q[k] = (x != x || x <= 0.0) ? 0ull : (x >= 2097151.0 ? 2097151ull : (uint64_t)x);
+        const double least = from_key(~bounds[k]);
+        const float ext = (float)(from_key(bounds[3 + k]) - least);
+        const float x = (float)(0.5 * (lo[k] + hi[k]) - least) * (2097152.f / ext);
+        q[k] = !(x > 0.f) ? 0ull : (x >= 2097151.f ? 2097151ull : (uint64_t)x);
     }
     keys[i] = (spread21(q[0]) << 2) | (spread21(q[1]) << 1) | spread21(q[2]);
     vals[i] = (int32_t)i;
-}
-
-__global__ void k_leaf_boxes(const double* __restrict__ aabbs, int64_t n, const int32_t* __restrict__ sorted,
-                             float4* __restrict__ leafbox) {
-    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    double lo[3], hi[3];
-    load_box(aabbs, sorted[p], lo, hi);
-    leafbox[2 * p] = make_float4(__double2float_rd(lo[0]), __double2float_rd(lo[1]), __double2float_rd(lo[2]), 0.f);
-    leafbox[2 * p + 1] =
-        make_float4(__double2float_ru(hi[0]), __double2float_ru(hi[1]), __double2float_ru(hi[2]), 0.f);
 }
 
 // common-prefix length of sorted keys i and j, ties broken by index
@@ -200,8 +198,8 @@ __device__ __forceinline__ int delta(const uint64_t* __restrict__ k, int64_t n, 
     return __clzll((long long)(a ^ b));
 }
 
-__global__ void k_karras(const uint64_t* __restrict__ k, int64_t n, int2* __restrict__ child, int2* __restrict__ range,
-                         int32_t* __restrict__ parent) {
+__global__ void k_karras(const uint64_t* __restrict__ k, int64_t n, uint32_t* __restrict__ parent,
+                         int32_t* __restrict__ visits) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n - 1) return;
     const int d = (delta(k, n, i, i + 1) - delta(k, n, i, i - 1)) > 0 ? 1 : -1;
@@ -222,42 +220,44 @@ __global__ void k_karras(const uint64_t* __restrict__ k, int64_t n, int2* __rest
     const int64_t lo = i < j ? i : j, hi = i < j ? j : i;
     const int left = lo == gamma ? ~(int)gamma : (int)gamma;
     const int right = hi == gamma + 1 ? ~(int)(gamma + 1) : (int)(gamma + 1);
-    child[i] = make_int2(left, right);
-    range[i] = make_int2((int)lo, (int)hi);
     const int64_t ni = n - 1;
-    parent[left >= 0 ? left : ni + ~left] = (int32_t)i;
-    parent[right >= 0 ? right : ni + ~right] = (int32_t)i;
+    parent[left >= 0 ? left : ni + ~left] = (uint32_t)(2 * i);
+    parent[right >= 0 ? right : ni + ~right] = (uint32_t)(2 * i + 1);
+    visits[i] = 0;
+    if (i == 0) parent[0] = kRoot;
 }
 
-__device__ __forceinline__ void child_box(const Tree& t, int c, float4& lo, float4& hi) {
-    if (c < 0) {
-        lo = t.leafbox[2 * (int64_t)~c];
-        hi = t.leafbox[2 * (int64_t)~c + 1];
-    } else {
-        lo = __ldcg(t.box + 2 * (int64_t)c);
-        hi = __ldcg(t.box + 2 * (int64_t)c + 1);
-    }
-}
-
-__global__ void k_refit(Tree t) {
+// The nodes' records, from the leaves up: every child writes its half of its
+// parent's record (box, id, last position), and the second one to arrive goes
+// on with the parent.
+__global__ void k_refit(const double* __restrict__ aabbs, Tree t) {
     int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= t.n) return;
-    const int64_t ni = t.n - 1;
-    int node = t.parent[ni + p];
+    const int leaf = t.sorted[p];
+    double dlo[3], dhi[3];
+    load_box(aabbs, leaf, dlo, dhi);
+    float4 lo = make_float4(__double2float_rd(dlo[0]), __double2float_rd(dlo[1]), __double2float_rd(dlo[2]),
+                            __int_as_float(~leaf));
+    float4 hi = make_float4(__double2float_ru(dhi[0]), __double2float_ru(dhi[1]), __double2float_ru(dhi[2]),
+                            __int_as_float((int)p));
+    uint32_t up = t.parent[t.n - 1 + p];
     int guard = 0;
-    while (node >= 0 && guard++ < 4 * kStack) {
+    while (up != kRoot && guard++ < 4 * kStack) {
+        const uint32_t side = up & 1, node = up >> 1;
+        float4* const rec = t.node[node].child;
+        __stcg(rec + 2 * side, lo);
+        __stcg(rec + 2 * side + 1, hi);
         __threadfence();
         if (atomicAdd(t.visits + node, 1) == 0) return;  // the sibling subtree is not done yet
-        int2 c = t.child[node];
-        float4 alo, ahi, blo, bhi;
-        child_box(t, c.x, alo, ahi);
-        child_box(t, c.y, blo, bhi);
-        __stcg(t.box + 2 * (int64_t)node, make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), 0.f));
-        __stcg(t.box + 2 * (int64_t)node + 1,
-               make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.f));
-        node = t.parent[node];
+        __threadfence();
+        t.visits[node] = 0;  // for the next refit
+        const float4 olo = __ldcg(rec + 2 * (1 - side)), ohi = __ldcg(rec + 2 * (1 - side) + 1);
+        lo = make_float4(fminf(lo.x, olo.x), fminf(lo.y, olo.y), fminf(lo.z, olo.z), __int_as_float((int)node));
+        hi = make_float4(fmaxf(hi.x, ohi.x), fmaxf(hi.y, ohi.y), fmaxf(hi.z, ohi.z),
+                         __int_as_float(max(__float_as_int(hi.w), __float_as_int(ohi.w))));
+        up = t.parent[node];
     }
-    if (node >= 0) atomicExch(t.flags, 1);
+    if (up != kRoot) atomicExch(t.flags, 1);
 }
 
 // ----------------------------------------------------------- queries
@@ -265,139 +265,136 @@ __device__ __forceinline__ bool overlap32(const float4& alo, const float4& ahi, 
     return alo.x <= bhi.x && ahi.x >= blo.x && alo.y <= bhi.y && ahi.y >= blo.y && alo.z <= bhi.z && ahi.z >= blo.z;
 }
 
-// aabb_tree.py:504-527, closed intervals
+// aabb_tree.py:504-527, closed intervals; the compares on integers (d3d_device.cuh)
 __device__ __forceinline__ bool overlap64(const double* a, const double* b) {
-    return a[0] <= b[1] && a[1] >= b[0] && a[2] <= b[3] && a[3] >= b[2] && a[4] <= b[5] && a[5] >= b[4];
+    return d3d::le(a[0], b[1]) && d3d::le(b[0], a[1]) && d3d::le(a[2], b[3]) && d3d::le(b[2], a[3]) &&
+           d3d::le(a[4], b[5]) && d3d::le(b[4], a[5]);
 }
 
-// warp-ballot compaction of one hit per lane
-__device__ __forceinline__ void emit(bool want, uint64_t key, unsigned long long* count, uint64_t* out,
-                                     int64_t cap) {
+// One hit each of the lanes that call it together: one atomic for all of them.
+__device__ __forceinline__ void emit(uint64_t key, unsigned long long* count, uint64_t* out, int64_t cap) {
     const unsigned active = __activemask();
-    const unsigned m = __ballot_sync(active, want);
-    if (!m) return;
     const int lane = threadIdx.x & 31;
-    const int leader = __ffs(m) - 1;
+    const int leader = __ffs(active) - 1;
     unsigned long long base = 0;
-    if (lane == leader) base = atomicAdd(count, (unsigned long long)__popc(m));
+    if (lane == leader) base = atomicAdd(count, (unsigned long long)__popc(active));
     base = __shfl_sync(active, base, leader);
-    if (want) {
-        unsigned long long idx = base + __popc(m & ((1u << lane) - 1u));
-        if ((int64_t)idx < cap) out[idx] = key;
+    const unsigned long long idx = base + __popc(active & ((1u << lane) - 1u));
+    if ((int64_t)idx < cap) out[idx] = key;
+}
+
+// One thread's walk of the tree for query box `box` (FP64) / qlo, qhi (FP32
+// outward): key_of(leaf) gives the key of each leaf whose exact box
+// overlaps it, subtrees that end at or before position `after` are skipped.
+// The FP32 boxes of the leaves are tested first: they hold the exact ones.
+template <typename Key>
+__device__ __forceinline__ void walk(const double* __restrict__ aabbs, const Tree& t, const double* box, float4 qlo,
+                                     float4 qhi, int after, Key key_of, unsigned long long* count, uint64_t* out,
+                                     int64_t cap) {
+    int stack[kStack];
+    int sp = 0;
+    int node = 0;
+    while (node >= 0) {
+        const float4* r = t.node[node].child;
+        const float4 rec[4] = {__ldg(r), __ldg(r + 1), __ldg(r + 2), __ldg(r + 3)};
+        int next = -1;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float4 lo = rec[2 * h], hi = rec[2 * h + 1];
+            if (__float_as_int(hi.w) <= after || !overlap32(qlo, qhi, lo, hi)) continue;
+            const int x = __float_as_int(lo.w);
+            if (x < 0) {
+                if (overlap64(box, aabbs + 6 * (int64_t)~x)) emit(key_of(~x), count, out, cap);
+            } else if (next < 0) {
+                next = x;  // walked next; the other child waits on the stack
+            } else if (sp < kStack) {
+                stack[sp++] = x;
+            } else {
+                atomicExch(reinterpret_cast<int*>(count + 1), 1);
+            }
+        }
+        node = next >= 0 ? next : (sp > 0 ? stack[--sp] : -1);
     }
 }
 
-// Self pairs: thread p (sorted position) reports every leaf q > p whose
-// exact box overlaps its own; subtrees whose sorted range ends at or before
-// p are skipped, so each unordered pair is found once.
-__global__ void k_self_pairs(const double* __restrict__ aabbs, Tree t, unsigned long long* count, uint64_t* out,
-                             int64_t cap) {
+// the refit's flag beside the count, so that one copy reads both
+__device__ __forceinline__ void pass_flags(const Tree& t, unsigned long long* count) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && t.flags[0]) atomicExch(reinterpret_cast<int*>(count + 1), 1);
+}
+
+__device__ __forceinline__ void outward(const double* box, float4& lo, float4& hi) {
+    lo = make_float4(__double2float_rd(box[0]), __double2float_rd(box[2]), __double2float_rd(box[4]), 0.f);
+    hi = make_float4(__double2float_ru(box[1]), __double2float_ru(box[3]), __double2float_ru(box[5]), 0.f);
+}
+
+// Pair keys: the first index above the `bits` of the second.
+// Self pairs: thread p (sorted position) reports every leaf after p whose
+// exact box overlaps its own, so each unordered pair is found once.
+__global__ void k_self_pairs(const double* __restrict__ aabbs, Tree t, int bits, unsigned long long* count,
+                             uint64_t* out, int64_t cap) {
+    pass_flags(t, count);
     int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= t.n - 1) return;  // the last leaf has no later leaves
     const int op = t.sorted[p];
     double box[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) box[k] = aabbs[6 * (int64_t)op + k];
-    const float4 qlo = t.leafbox[2 * p], qhi = t.leafbox[2 * p + 1];
-    int stack[kStack];
-    int sp = 0;
-    stack[sp++] = 0;
-    while (sp > 0) {
-        const int node = stack[--sp];
-        const int2 c = t.child[node];
-        const int cc[2] = {c.x, c.y};
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int x = cc[h];
-            bool hit = false;
-            uint64_t key = 0;
-            if (x < 0) {
-                const int64_t q = ~x;
-                if (q > p) {
-                    const int oq = t.sorted[q];
-                    if (overlap64(box, aabbs + 6 * (int64_t)oq)) {
-                        hit = true;
-                        const uint32_t a = (uint32_t)min(op, oq), b = (uint32_t)max(op, oq);
-                        key = ((uint64_t)a << 32) | b;
-                    }
-                }
-            } else if (t.range[x].y > p && overlap32(qlo, qhi, t.box[2 * (int64_t)x], t.box[2 * (int64_t)x + 1])) {
-                if (sp < kStack)
-                    stack[sp++] = x;
-                else
-                    atomicExch(t.flags + 1, 1);
-            }
-            emit(hit, key, count, out, cap);
-        }
-    }
+    float4 qlo, qhi;
+    outward(box, qlo, qhi);
+    walk(aabbs, t, box, qlo, qhi, (int)p,
+         [=](int leaf) { return ((uint64_t)(uint32_t)min(op, leaf) << bits) | (uint32_t)max(op, leaf); }, count, out,
+         cap);
 }
 
 // Box queries: thread q reports every leaf whose exact box overlaps query q.
 __global__ void k_query_boxes(const double* __restrict__ aabbs, Tree t, const double* __restrict__ boxes, int64_t m,
-                              unsigned long long* count, uint64_t* out, int64_t cap) {
+                              int bits, unsigned long long* count, uint64_t* out, int64_t cap) {
+    pass_flags(t, count);
     int64_t qi = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (qi >= m) return;
     double box[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) box[k] = boxes[6 * qi + k];
-    const float4 qlo = make_float4(__double2float_rd(box[0]), __double2float_rd(box[2]), __double2float_rd(box[4]), 0.f);
-    const float4 qhi = make_float4(__double2float_ru(box[1]), __double2float_ru(box[3]), __double2float_ru(box[5]), 0.f);
+    auto key_of = [=](int leaf) { return ((uint64_t)(uint32_t)leaf << bits) | (uint32_t)qi; };
     if (t.n == 1) {
-        const bool hit = overlap64(box, aabbs + 6 * (int64_t)t.sorted[0]);
-        emit(hit, ((uint64_t)(uint32_t)t.sorted[0] << 32) | (uint32_t)qi, count, out, cap);
+        const int leaf = t.sorted[0];
+        if (overlap64(box, aabbs + 6 * (int64_t)leaf)) emit(key_of(leaf), count, out, cap);
         return;
     }
-    int stack[kStack];
-    int sp = 0;
-    stack[sp++] = 0;
-    while (sp > 0) {
-        const int node = stack[--sp];
-        const int2 c = t.child[node];
-        const int cc[2] = {c.x, c.y};
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int x = cc[h];
-            bool hit = false;
-            uint64_t key = 0;
-            if (x < 0) {
-                const int ol = t.sorted[~x];
-                if (overlap64(box, aabbs + 6 * (int64_t)ol)) {
-                    hit = true;
-                    key = ((uint64_t)(uint32_t)ol << 32) | (uint32_t)qi;
-                }
-            } else if (overlap32(qlo, qhi, t.box[2 * (int64_t)x], t.box[2 * (int64_t)x + 1])) {
-                if (sp < kStack)
-                    stack[sp++] = x;
-                else
-                    atomicExch(t.flags + 1, 1);
-            }
-            emit(hit, key, count, out, cap);
-        }
-    }
+    float4 qlo, qhi;
+    outward(box, qlo, qhi);
+    walk(aabbs, t, box, qlo, qhi, -1, key_of, count, out, cap);
 }
 
-__global__ void k_decode(const uint64_t* __restrict__ keys, int64_t n, int32_t* __restrict__ pairs) {
+__global__ void k_decode(const uint64_t* __restrict__ keys, int64_t n, int bits, int32_t* __restrict__ pairs) {
     int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    uint64_t v = keys[k];
-    pairs[2 * k] = (int32_t)(v >> 32);
-    pairs[2 * k + 1] = (int32_t)(v & 0xffffffffu);
+    const uint64_t v = keys[k];
+    pairs[2 * k] = (int32_t)(v >> bits);
+    pairs[2 * k + 1] = (int32_t)(v & ((1ull << bits) - 1));
+}
+
+// bits that hold 0 .. n-1
+int index_bits(int64_t n) {
+    int b = 1;
+    while ((int64_t(1) << b) < n) ++b;
+    return b;
 }
 
 // Sort the hit keys and write int32 pairs; synchronises to read the count.
 int finish_pairs(unsigned long long* d_count, uint64_t* keys, uint64_t* keys_alt, void* cub_temp, size_t cub_bytes,
-                 int32_t* pairs, int64_t capacity, int64_t* n_pairs, const int32_t* flags, cudaStream_t st) {
-    unsigned long long count = 0;
-    int hflags[2] = {0, 0};
-    cudaMemcpyAsync(&count, d_count, sizeof(count), cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(hflags, flags, sizeof(hflags), cudaMemcpyDeviceToHost, st);
+                 int32_t* pairs, int64_t capacity, int64_t* n_pairs, int bits_first, int bits_second, cudaStream_t st) {
+    // the pair count and the error flag
+    unsigned long long read[2] = {0, 0};
+    cudaMemcpyAsync(read, d_count, sizeof(read), cudaMemcpyDeviceToHost, st);
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
         d3d::set_error("bvh query: %s", cudaGetErrorString(e));
         return D3D_ERR_CUDA;
     }
+    const unsigned long long count = read[0];
     if (n_pairs) *n_pairs = (int64_t)count;
-    if (hflags[0] || hflags[1]) {
+    if (read[1]) {
         d3d::set_error("bvh: traversal stack or refit bound exceeded (tree deeper than %d)", kStack);
         return D3D_ERR_CAPACITY;
     }
@@ -406,18 +403,20 @@ int finish_pairs(unsigned long long* d_count, uint64_t* keys, uint64_t* keys_alt
         return D3D_ERR_CAPACITY;
     }
     if (count == 0) return D3D_SUCCESS;
+    // the keys' used bits only: a pass per 8 bits (5 instead of 8 below 2^20 boxes)
+    const int bits = bits_first + bits_second;
     size_t need = 0;
-    cub::DeviceRadixSort::SortKeys(nullptr, need, keys, keys_alt, (int)count, 0, 64, st);
+    cub::DeviceRadixSort::SortKeys(nullptr, need, keys, keys_alt, (int)count, 0, bits, st);
     if (need > cub_bytes) {
         d3d::set_error("bvh query: sort temporary storage too small");
         return D3D_ERR_CAPACITY;
     }
-    e = cub::DeviceRadixSort::SortKeys(cub_temp, need, keys, keys_alt, (int)count, 0, 64, st);
+    e = cub::DeviceRadixSort::SortKeys(cub_temp, need, keys, keys_alt, (int)count, 0, bits, st);
     if (e != cudaSuccess) {
         d3d::set_error("bvh query: sort failed: %s", cudaGetErrorString(e));
         return D3D_ERR_CUDA;
     }
-    k_decode<<<d3d::grid_for((int64_t)count, kBlock), kBlock, 0, st>>>(keys_alt, (int64_t)count, pairs);
+    k_decode<<<d3d::grid_for((int64_t)count, kBlock), kBlock, 0, st>>>(keys_alt, (int64_t)count, bits_second, pairs);
     return d3d::check_launch("bvh query");
 }
 
@@ -446,14 +445,12 @@ extern "C" int d3d_bvh_build(const double* aabbs, int64_t n, void* tree, size_t 
     Tree t;
     layout(tree, n, &t);
     cudaStream_t st = d3d::as_stream(stream);
-    cudaMemsetAsync(t.flags, 0, 4 * sizeof(int32_t), st);
+    cudaMemsetAsync(t.flags, 0, 256, st);  // the bounds' keys with them
     if (n == 0) return d3d::check_launch("d3d_bvh_build");
     D3D_REQUIRE(aabbs, "d3d_bvh_build: null aabbs");
-    int blocks = (int)((n + kBlock - 1) / kBlock);
-    if (blocks > kBoundBlocks) blocks = kBoundBlocks;
-    k_center_bounds<<<blocks, kBlock, 0, st>>>(aabbs, n, t.bounds + 6);
-    k_reduce_bounds<<<1, 32, 0, st>>>(t.bounds + 6, blocks, t.bounds);
-    k_morton<<<d3d::grid_for(n, kBlock), kBlock, 0, st>>>(aabbs, n, t.bounds, t.keys, t.vals);
+    const unsigned blocks = d3d::grid_for(n, kBlock);
+    k_center_bounds<<<blocks < 304 ? blocks : 304, kBlock, 0, st>>>(aabbs, n, t.bounds);
+    k_morton<<<blocks, kBlock, 0, st>>>(aabbs, n, t.bounds, t.keys, t.vals);
     size_t cub_bytes = t.cub_bytes;
     cudaError_t e = cub::DeviceRadixSort::SortPairs(t.cub_temp, cub_bytes, t.keys, t.keys_out, t.vals, t.sorted, (int)n,
                                                     0, 63, st);
@@ -461,12 +458,9 @@ extern "C" int d3d_bvh_build(const double* aabbs, int64_t n, void* tree, size_t 
         d3d::set_error("d3d_bvh_build: sort failed: %s", cudaGetErrorString(e));
         return D3D_ERR_CUDA;
     }
-    k_leaf_boxes<<<d3d::grid_for(n, kBlock), kBlock, 0, st>>>(aabbs, n, t.sorted, t.leafbox);
     if (n > 1) {
-        cudaMemsetAsync(t.parent, 0xff, sizeof(int32_t) * (size_t)(2 * n - 1), st);
-        cudaMemsetAsync(t.visits, 0, sizeof(int32_t) * (size_t)(n - 1), st);
-        k_karras<<<d3d::grid_for(n - 1, kBlock), kBlock, 0, st>>>(t.keys_out, n, t.child, t.range, t.parent);
-        k_refit<<<d3d::grid_for(n, kBlock), kBlock, 0, st>>>(t);
+        k_karras<<<d3d::grid_for(n - 1, kBlock), kBlock, 0, st>>>(t.keys_out, n, t.parent, t.visits);
+        k_refit<<<blocks, kBlock, 0, st>>>(aabbs, t);
     }
     return d3d::check_launch("d3d_bvh_build");
 }
@@ -485,11 +479,7 @@ extern "C" int d3d_bvh_refit(const double* aabbs, int64_t n, void* tree, size_t 
     layout(tree, n, &t);
     cudaStream_t st = d3d::as_stream(stream);
     // same leaf order and topology; the boxes of leaves and nodes are redone
-    k_leaf_boxes<<<d3d::grid_for(n, kBlock), kBlock, 0, st>>>(aabbs, n, t.sorted, t.leafbox);
-    if (n > 1) {
-        cudaMemsetAsync(t.visits, 0, sizeof(int32_t) * (size_t)(n - 1), st);
-        k_refit<<<d3d::grid_for(n, kBlock), kBlock, 0, st>>>(t);
-    }
+    if (n > 1) k_refit<<<d3d::grid_for(n, kBlock), kBlock, 0, st>>>(aabbs, t);
     return d3d::check_launch("d3d_bvh_refit");
 }
 
@@ -529,14 +519,15 @@ extern "C" int d3d_bvh_self_pairs(const double* aabbs, int64_t n, const void* tr
     int rc = query_common(tree, n, capacity, scratch, scratch_bytes, &t, &count, &keys, &alt, &cub_temp, &cub_bytes);
     if (rc) return rc;
     cudaStream_t st = d3d::as_stream(stream);
-    cudaMemsetAsync(count, 0, sizeof(unsigned long long), st);
+    cudaMemsetAsync(count, 0, 2 * sizeof(unsigned long long), st);
+    const int bits = index_bits(n);
     if (n > 1) {
         D3D_REQUIRE(aabbs && (pairs || capacity == 0), "d3d_bvh_self_pairs: null pointer");
-        k_self_pairs<<<d3d::grid_for(n - 1, 128), 128, 0, st>>>(aabbs, t, count, keys, capacity);
+        k_self_pairs<<<d3d::grid_for(n - 1, 128), 128, 0, st>>>(aabbs, t, bits, count, keys, capacity);
         rc = d3d::check_launch("d3d_bvh_self_pairs");
         if (rc) return rc;
     }
-    return finish_pairs(count, keys, alt, cub_temp, cub_bytes, pairs, capacity, n_pairs, t.flags, st);
+    return finish_pairs(count, keys, alt, cub_temp, cub_bytes, pairs, capacity, n_pairs, bits, bits, st);
 }
 
 extern "C" int d3d_bvh_query(const double* aabbs, int64_t n, const void* tree, const double* boxes, int64_t m,
@@ -551,12 +542,13 @@ extern "C" int d3d_bvh_query(const double* aabbs, int64_t n, const void* tree, c
     if (rc) return rc;
     D3D_REQUIRE(m >= 0 && m < (int64_t(1) << 31), "d3d_bvh_query: m out of range");
     cudaStream_t st = d3d::as_stream(stream);
-    cudaMemsetAsync(count, 0, sizeof(unsigned long long), st);
+    cudaMemsetAsync(count, 0, 2 * sizeof(unsigned long long), st);
+    const int bits = index_bits(m);
     if (n > 0 && m > 0) {
         D3D_REQUIRE(aabbs && boxes && (pairs || capacity == 0), "d3d_bvh_query: null pointer");
-        k_query_boxes<<<d3d::grid_for(m, 128), 128, 0, st>>>(aabbs, t, boxes, m, count, keys, capacity);
+        k_query_boxes<<<d3d::grid_for(m, 128), 128, 0, st>>>(aabbs, t, boxes, m, bits, count, keys, capacity);
         rc = d3d::check_launch("d3d_bvh_query");
         if (rc) return rc;
     }
-    return finish_pairs(count, keys, alt, cub_temp, cub_bytes, pairs, capacity, n_pairs, t.flags, st);
+    return finish_pairs(count, keys, alt, cub_temp, cub_bytes, pairs, capacity, n_pairs, index_bits(n), bits, st);
 }
