@@ -162,8 +162,7 @@ class SelfCollisionBatch:
             base = torch.arange(self.n_configs, dtype=torch.int64, device=dev)[:, None] * nb
             self.i1 = (base + t(table[:, 0], torch.int64)[None, :]).reshape(-1).to(torch.int32).contiguous()
             self.i2 = (base + t(table[:, 1], torch.int64)[None, :]).reshape(-1).to(torch.int32).contiguous()
-            self._pa = t(table[:, 0], torch.int64)
-            self._pb = t(table[:, 1], torch.int64)
+            self._table = t(table, torch.int32)
             self.n_pairs = self.i1.numel()
             self.q = torch.zeros((self.n_configs, arm.dof), dtype=torch.float64, device=dev)
             self.poses = torch.empty((self.n_configs * nb, 12), dtype=torch.float64, device=dev)
@@ -208,12 +207,8 @@ class SelfCollisionBatch:
                                    _ptr(o["epa_status"]), _ptr(o["n_faces"]), _ptr(self.scratch),
                                    self.scratch.numel(), s))
         # contacts[c, body] = the body touches any listed partner (detect, self_collision.py:5-37)
-        hit = (o["dist"] == 0.0).view(self.n_configs, self.n_pair_types)
-        self.contacts.zero_()
-        self.contacts.index_put_((torch.arange(self.n_configs, device=self.device)[:, None], self._pa[None, :]),
-                                 hit, accumulate=True)
-        self.contacts.index_put_((torch.arange(self.n_configs, device=self.device)[:, None], self._pb[None, :]),
-                                 hit, accumulate=True)
+        _lib.check(lib.d3d_chain_contacts(_ptr(o["dist"]), self.n_configs, _ptr(self._table), self.n_pair_types,
+                                          self.arm.n_bodies, _ptr(self.contacts), s))
 
     def run(self, q, sync=True):
         """Check configurations q (n_configs, dof); returns the outputs as

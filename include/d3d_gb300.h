@@ -297,6 +297,13 @@ typedef struct {
  * self_collision.detect relies on, self_collision.py:5-64). */
 int d3d_chain_fk(const d3d_chain* chain, const double* q, int64_t n_configs, double* poses, void* stream);
 
+/* Contact flags of a batch of configurations: contacts[c][b] = 1 if body b is
+ * in a listed pair whose distance dist[c][p] is 0, else 0.  pairs[p] are two
+ * body indices (entries outside [0, n_bodies) are skipped).  The flags
+ * self_collision.detect returns per collider frame (self_collision.py:5-37). */
+int d3d_chain_contacts(const double* dist, int64_t n_configs, const int32_t* pairs, int64_t n_pairs, int32_t n_bodies,
+                       uint8_t* contacts, void* stream);
+
 /* Launch parameters of the batch kernels (process-wide, per library load).
  * gjk_block: threads per block of the GJK kernels (64, 128 or 256; the
  * plain FP64 GJK, whose blocks solve their simplices together, runs 128 for
