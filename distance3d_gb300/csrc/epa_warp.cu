@@ -718,26 +718,102 @@ __global__ void __launch_bounds__(32 * WARPS, kWarpsPerSm<T> / WARPS) k_epa_warp
     }
 }
 
-// The FP64 refinement of the FP32 search's converged faces (refine_face),
-// one pair per thread: the normal the search left in mtv, renormalised in
-// FP64, and mtv = n (n . w(n)) with RefineSupport.  In the search kernel the
-// whole warp waited on each pair's FP64 support chain.
+// The FP64 refinement of the FP32 search's converged faces (refine_face): the
+// normal the search left in mtv, renormalised in FP64, and mtv = n (n . w(n))
+// with RefineSupport.  In the search kernel the whole warp waited on each
+// pair's FP64 support chain.  A block lists the two supports of its pairs by
+// collider type (typelist.cuh); with a pair per thread the lanes of a warp ran
+// through all types (6.3 lanes per FP64 instruction).  Converged pairs of the
+// bench workload (310k): 210 -> 110 us.
+constexpr int kRefine = 128;
+
 template <bool MESH>
-__global__ void __launch_bounds__(128) k_epa_refine(d3d_store st, const int32_t* __restrict__ i1,
-                                                    const int32_t* __restrict__ i2, const int32_t* __restrict__ list,
-                                                    const unsigned long long* __restrict__ n_dev,
-                                                    double* __restrict__ mtv) {
+__global__ void __launch_bounds__(kRefine) k_epa_refine(d3d_store st, const int32_t* __restrict__ i1,
+                                                        const int32_t* __restrict__ i2,
+                                                        const int32_t* __restrict__ list,
+                                                        const unsigned long long* __restrict__ n_dev,
+                                                        double* __restrict__ mtv) {
+    __shared__ double dir[3 * kRefine], sup[2][3 * kRefine];
+    __shared__ int col[2 * kRefine];
+    __shared__ unsigned short task[2 * kRefine];  // thread << 1 | side
+    __shared__ int cnt[kSupportBins], next;
     const int64_t n = (int64_t)*n_dev;
-    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t k = list[j];
-        d3 nrm = mk(mtv[3 * k], mtv[3 * k + 1], mtv[3 * k + 2]);
-        nrm = nrm * (1.0 / sqrt(dot(nrm, nrm)));
-        d3 p, q;
-        pair_supports<double, RefineSupportT<MESH>>(st, i1[k], i2[k], nrm, p, q);
-        const d3 m = nrm * dot(p - q, nrm);
-        mtv[3 * k] = m.x;
-        mtv[3 * k + 1] = m.y;
-        mtv[3 * k + 2] = m.z;
+    const int t = threadIdx.x, ln = lane_id();
+    // fewer pairs per block where full blocks would leave SMs idle
+    const int64_t share = (n + gridDim.x - 1) / gridDim.x;
+    const int per = share < 16 ? 16 : (share > kRefine ? kRefine : (int)share);
+    for (int64_t base = (int64_t)blockIdx.x * per; base < n; base += (int64_t)gridDim.x * per) {
+        __syncthreads();  // the last round's reads
+        if (t < kSupportBins) cnt[t] = 0;
+        if (t == kSupportBins) next = 0;
+        __syncthreads();
+        const bool on = t < per && base + t < n;
+        int64_t k = 0;
+        d3 nrm = mk(0.0, 0.0, 0.0);
+        int bin[2] = {0, 0}, pos[2] = {0, 0};
+        if (on) {
+            k = list[base + t];
+            nrm = mk(mtv[3 * k], mtv[3 * k + 1], mtv[3 * k + 2]);
+            nrm = nrm * (1.0 / sqrt(dot(nrm, nrm)));
+            dir[t] = nrm.x;
+            dir[kRefine + t] = nrm.y;
+            dir[2 * kRefine + t] = nrm.z;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int c = (h ? i2 : i1)[k];
+                col[h * kRefine + t] = c;
+                const int4 m = __ldg(reinterpret_cast<const int4*>(st.meta) + c);
+                bin[h] = m.x == D3D_HULL ? kSearchBin : support_bin(m.x, m.w);
+                pos[h] = atomicAdd(cnt + bin[h], 1);
+            }
+        }
+        __syncthreads();
+        const Chunks ch = chunks_of(cnt, kSupportBins, ln == kSearchBin ? 4 : 32);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int p = ch.start(bin[h]) + pos[h];
+            if (on) task[p] = (unsigned short)(2 * t + h);
+        }
+        __syncthreads();
+        int cb, first, num;
+        while (ch.take(&next, cb, first, num)) {
+            const bool mine = ln < num;
+            const int e = task[first + (mine ? ln : 0)];
+            const int u = e >> 1, h = e & 1;
+            const int c = col[h * kRefine + u];
+            d3 d = mk(dir[u], dir[kRefine + u], dir[2 * kRefine + u]);
+            if (h) d = -d;
+            int vi = -1;
+            const f3 f = RefineSupportT<MESH>::rounded(d);
+            if (cb == kSearchBin) {  // the hulls, each by the whole warp
+                int type, nv, off;
+                load_meta(st, c, type, nv, off);
+                for (int q = 0; q < num; ++q) {
+                    const int w = warp_hull_argmax(
+                        st.verts32, __shfl_sync(kFull, off, q), max(__shfl_sync(kFull, nv, q), 1),
+                        mk(__shfl_sync(kFull, f.x, q), __shfl_sync(kFull, f.y, q), __shfl_sync(kFull, f.z, q)));
+                    if (ln == q) vi = w;
+                }
+            }
+            if (mine) {
+                Col<double> cl;
+                load_col(st, c, cl);
+                const d3 x = RefineSupportT<MESH>::eval_at(cl, st, d, f, vi);
+                sup[h][u] = x.x;
+                sup[h][kRefine + u] = x.y;
+                sup[h][2 * kRefine + u] = x.z;
+            }
+            __syncwarp();
+        }
+        __syncthreads();
+        if (on) {
+            const d3 p = mk(sup[0][t], sup[0][kRefine + t], sup[0][2 * kRefine + t]);
+            const d3 q = mk(sup[1][t], sup[1][kRefine + t], sup[1][2 * kRefine + t]);
+            const d3 m = nrm * dot(p - q, nrm);
+            mtv[3 * k] = m.x;
+            mtv[3 * k + 1] = m.y;
+            mtv[3 * k + 2] = m.z;
+        }
     }
 }
 
@@ -768,7 +844,7 @@ int launch_warp(const d3d_store& store, const int32_t* i1, const int32_t* i2, co
     int rc = check_launch("d3d_epa (mixed)");
     if (rc || !refine) return rc;
     const void* kr = (const void*)k_epa_refine<MESH>;
-    k_epa_refine<MESH><<<persistent_blocks(kr, 128, n), 128, 0, stream>>>(store, i1, i2, refine, n_refine, mtv);
+    k_epa_refine<MESH><<<persistent_blocks(kr, kRefine, 8 * n), kRefine, 0, stream>>>(store, i1, i2, refine, n_refine, mtv);
     return check_launch("d3d_epa (mixed, refinement)");
 }
 

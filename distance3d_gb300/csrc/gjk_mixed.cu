@@ -7,9 +7,9 @@
 //    closest point and the search direction of each final simplex row on
 //    (80 bytes/pair) and appends clipped and unconverged pairs to the
 //    fallback list.
-// R  (the refinement pass) takes one warp per 32 consecutive slots of the
-//    type-sorted order, so that a warp's lanes evaluate the same supports.
-//    Each lane re-evaluates its pair's final simplex rows in FP64 along their
+// R  (the refinement pass) lists the rows of a block's pairs by collider type,
+//    so that a warp's lanes evaluate the same supports.
+//    The final simplex rows are re-evaluated in FP64 along their
 //    FP32 directions (polytope supports choose their vertex by an FP32 argmax
 //    and return the FP64 vertex) and, for a separated pair, one more support
 //    pair along -v, the closest point A ended on.  A separated pair whose
@@ -75,12 +75,69 @@ struct Lists {
 // slots a warp claims from the type-sorted order at a time
 constexpr int kChunk = 32;
 
+// Lanes per warp that take pairs where n pairs are spread over the whole grid.
+__device__ __forceinline__ long long spread_lanes(long long n, int block) {
+    const long long warps = (long long)gridDim.x * (block / 32);
+    return n >= 32 * warps ? 32 : (n + warps - 1) / warps;
+}
+
 // Phase A's register budget: 16 resident warps per SM (128 registers), its
 // simplex P/Q rows in shared memory (ARows).  At 1M pairs: 3.9 ms for the
 // mixed GJK, against 4.2 with 12 warps and the rows in registers, 4.2 with 20
 // warps and 4.9 with 24 (more spilled registers).
 template <int BLOCK>
 constexpr int phase_a_min_blocks() { return 512 / BLOCK; }
+
+// A batch that does not fill the grid (spread_lanes below) runs in
+// k_gjk_mixed_a_spread: a few lanes of every warp take pairs, so that their
+// different supports and simplex sizes cost little, and the others help to
+// scan their hulls.  3,000 six-type pairs: 203 -> 91 us; a full grid stays
+// with k_gjk_mixed_a (1M pairs: 2.09 ms, 2.36 in the spread form).
+template <int BLOCK, bool MESH>
+__global__ void __launch_bounds__(BLOCK, phase_a_min_blocks<BLOCK>()) k_gjk_mixed_a_spread(
+    d3d_store s, const int32_t* __restrict__ i1, const int32_t* __restrict__ i2, const int32_t* __restrict__ order,
+    int64_t n, const int64_t* __restrict__ n_dev, float tol_sq, float max_d2, int max_iter,
+    Handoff* __restrict__ hand, DistanceOut out, Lists lists) {
+    constexpr unsigned kAll = 0xffffffffu;
+    if (n_dev) n = *n_dev;
+    __shared__ float4 arows[4 * BLOCK];
+    PhaseALoop<ARows<BLOCK>> L;
+    L.S.R.base = arows + threadIdx.x;
+    int64_t pid = 0;
+    int a = 0, b = 0;
+    const long long lanes = spread_lanes(n, BLOCK);
+    bool have = false, bad = false, exhausted = (int)(threadIdx.x & 31) >= lanes;
+    WarpChunk chunk;
+    while (true) {
+        __syncwarp();
+        const bool want = !have && !exhausted;
+        const long long slot = fetch_slot_chunked(lists.ctr + kCurA, want, chunk, kAll, kChunk, 0);
+        if (want) {
+            if (slot >= n) {
+                exhausted = true;
+            } else {
+                pid = order ? order[slot] : slot;
+                a = i1[pid];
+                b = i2[pid];
+                bad = !pair_ok(s, a, b);
+                pa_begin(L);
+                have = true;
+            }
+        }
+        if (!__any_sync(kAll, have)) break;
+        int o = pa_step<MESH, true>(L, have && !bad, s, a, b, tol_sq, max_d2, max_iter);
+        if (have && bad) o = PA_BAD_INDEX;
+        const bool done = have && o >= 0;
+        if (done) {
+            hand[pid] = pa_handoff(L, o);
+            if (bad) store_bad_index(out, pid);
+            have = false;
+        }
+        __syncwarp();
+        append_lanes(kAll, lists.fallback, lists.ctr + kNumFallback, done && (o == PA_CLIPPED || o == PA_FAILED),
+                     (int32_t)pid);
+    }
+}
 
 template <int BLOCK, bool MESH>
 __global__ void __launch_bounds__(BLOCK, phase_a_min_blocks<BLOCK>()) k_gjk_mixed_a(d3d_store s, const int32_t* __restrict__ i1,
@@ -118,7 +175,7 @@ __global__ void __launch_bounds__(BLOCK, phase_a_min_blocks<BLOCK>()) k_gjk_mixe
         __syncwarp(live);  // the round starts converged (pa_step keeps it so through the solve)
         // a pair with an out-of-range index ends at once; R skips it (its outcome is neither
         // separated nor touching) and it joins no list
-        const int o = bad ? PA_BAD_INDEX : pa_step<MESH>(L, s, a, b, tol_sq, max_d2, max_iter);
+        const int o = bad ? PA_BAD_INDEX : pa_step<MESH, false>(L, true, s, a, b, tol_sq, max_d2, max_iter);
         const bool done = o >= 0;
         if (done) {
             hand[pid] = pa_handoff(L, o);
@@ -233,17 +290,24 @@ __device__ __forceinline__ void r_finish(const double* my, int nr, bool sep, boo
     lists.run_pid[slot] = pid;
 }
 
-// R, one lane per slot of the order (see the top of this file).  The grid
-// covers the capacity; slots at and beyond the pair count are flagged 0.
-// Each lane evaluates its pair's FP64 rows; the checks that follow run in
-// different branches for touching pairs and for separated pairs of one, two
-// and three rows, so the block regroups them: the pairs are sorted by that
-// class (counting sort over the block, the rows staying where they are in
-// shared memory) and thread t runs the t-th pair's checks (r_finish).
+// R, one lane per slot of the order (see the top of this file), `per` slots
+// per block.  The grid covers the capacity; slots at and beyond the pair count
+// are flagged 0.  The block lists every row's two supports by collider type
+// (typelist.cuh) and its warps evaluate them 32 of a type at a time, the hulls
+// of the gap rows, whose vertex has to be searched, one per warp.  (One lane
+// per pair evaluated its rows in turn: 20 lanes per FP64 instruction in the
+// type-sorted order, 8.6 in a batch too small to be sorted.  1M pairs 1.00 ->
+// 0.86 ms, 300,032 robot pairs 270 -> 187 us, 3,000 pairs 65 -> 20 us.)  The checks that
+// follow run in different branches for touching pairs and for separated pairs
+// of one, two and three rows, so the block regroups them: the pairs are sorted
+// by that class (counting sort over the block, the rows staying where they are
+// in shared memory) and thread t runs the t-th pair's checks (r_finish).
+constexpr int kRowTasks = 10;  // rows x sides of a pair
+
 template <int BLOCK, bool MESH>
 __global__ void __launch_bounds__(BLOCK) k_gjk_mixed_r(d3d_store s, const int32_t* __restrict__ i1,
                                                         const int32_t* __restrict__ i2,
-                                                        const int32_t* __restrict__ order, int64_t cap,
+                                                        const int32_t* __restrict__ order, int64_t cap, int per,
                                                         const int64_t* __restrict__ n_dev, d3d_gjk_options opt,
                                                         const Handoff* __restrict__ hand, DistanceOut o, Lists lists) {
     constexpr int W = BLOCK / 32;
@@ -252,15 +316,22 @@ __global__ void __launch_bounds__(BLOCK) k_gjk_mixed_r(d3d_store s, const int32_
     __shared__ double rows[30 * BLOCK];
     __shared__ float4 tv[BLOCK];       // the handoff's v of each lane's pair
     __shared__ int tpid[BLOCK], tita[BLOCK], tcls[BLOCK];
+    __shared__ int col[2 * BLOCK];
+    __shared__ unsigned short list[kRowTasks * BLOCK];  // thread * kRowTasks + 2 row + side
+    __shared__ int tcnt[kSupportBins], next;
     __shared__ unsigned short tperm[BLOCK];
     __shared__ int cnt[4 * W];
     const int64_t n = n_dev ? *n_dev : cap;
-    const int64_t slot = (int64_t)blockIdx.x * BLOCK + threadIdx.x;
+    const int64_t slot0 = (int64_t)blockIdx.x * per;
+    const int64_t slot = slot0 + threadIdx.x;
+    const bool in = (int)threadIdx.x < per && slot < cap;
     const int ln = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    if (threadIdx.x < kSupportBins) tcnt[threadIdx.x] = 0;
+    if (threadIdx.x == kSupportBins) next = 0;
     int32_t pid = 0;
     int outcome = PA_FAILED, nr = 0, it_a = 0;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (slot < n && slot < cap) {
+    if (in && slot < n) {
         pid = order ? order[slot] : (int32_t)slot;
         v = hand[pid].v;
         outcome = __float_as_int(v.w) & 0xff;
@@ -271,48 +342,78 @@ __global__ void __launch_bounds__(BLOCK) k_gjk_mixed_r(d3d_store s, const int32_
     const bool rows_ok = mine && nr >= 1 && nr <= 4;
     const bool sep = rows_ok && outcome == PA_SEPARATED && nr <= 3;
     const bool touch = rows_ok && outcome == PA_TOUCHING && nr == 4;
-    int a = 0, b = 0;
-    if (rows_ok) {
-        a = i1[pid];
-        b = i2[pid];
-    }
     // the rows in FP64, then the gap row of a separated pair along -v
     const int count = rows_ok ? nr + (sep ? 1 : 0) : 0;
     double* my = rows + threadIdx.x;
-#pragma unroll 1
-    for (int j = 0; j < 5; ++j) {
-        if (j < count) {
-            d3 d;
-            float4 f = make_float4(0.f, 0.f, 0.f, __uint_as_float(0xffffffffu));  // the gap row: no vertices known
-            if (j < nr) {
-                f = hand[pid].d[j];
-                d = mk((double)f.x, (double)f.y, (double)f.z);
-            } else {
-                d = mk(-(double)v.x, -(double)v.y, -(double)v.z);
-            }
-            // the polytope vertices phase A took along this row's direction are read, not searched again
-            d3 p, q;
-#pragma unroll 1
-            for (int k = 0; k < 2; ++k) {
-                Col<double> c;
-                load_col(s, k ? b : a, c);
-                const d3 x = RefineSupportT<MESH>::eval_at(c, s, k ? -d : d, handoff_vertex(f, k));
-                if (k)
-                    q = x;
-                else
-                    p = x;
-            }
-            my[(6 * j + 0) * BLOCK] = p.x;
-            my[(6 * j + 1) * BLOCK] = p.y;
-            my[(6 * j + 2) * BLOCK] = p.z;
-            my[(6 * j + 3) * BLOCK] = q.x;
-            my[(6 * j + 4) * BLOCK] = q.y;
-            my[(6 * j + 5) * BLOCK] = q.z;
+    tv[threadIdx.x] = v;
+    tpid[threadIdx.x] = pid;
+    __syncthreads();
+    int bin[2] = {0, 0}, pos[2] = {0, 0}, found[2] = {0, 0};
+    bool search[2] = {false, false};
+    if (rows_ok) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int c = (k ? i2 : i1)[pid];
+            col[k * BLOCK + threadIdx.x] = c;
+            const int4 m = __ldg(reinterpret_cast<const int4*>(s.meta) + c);
+            bin[k] = support_bin(m.x, m.w);
+            search[k] = sep && m.x == D3D_HULL;
+            pos[k] = atomicAdd(tcnt + bin[k], search[k] ? count - 1 : count);
+            if (search[k]) found[k] = atomicAdd(tcnt + kSearchBin, 1);
         }
     }
+    __syncthreads();
+    const Chunks ch = chunks_of(tcnt, kSupportBins, ln == kSearchBin ? 2 : 32);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int p0 = ch.start(bin[k]) + pos[k], p1 = ch.start(kSearchBin) + found[k];
+        const unsigned short t = (unsigned short)(threadIdx.x * kRowTasks + k);
+        for (int j = 0; j < (search[k] ? count - 1 : count); ++j) list[p0 + j] = t + 2 * j;
+        if (search[k]) list[p1] = t + 2 * nr;
+    }
+    __syncthreads();
+    int cb, first, num;
+    while (ch.take(&next, cb, first, num)) {
+        // the hulls to search, each by the whole warp
+        int vi = -1;
+        const bool on = ln < num;
+        const int e = list[first + (on ? ln : 0)];
+        const int t = e / kRowTasks, j = (e % kRowTasks) >> 1, k = e & 1;
+        const int c = col[k * BLOCK + t];
+        const float4 u = tv[t];
+        const int rn = (__float_as_int(u.w) >> 8) & 0xff;
+        float4 f = make_float4(-u.x, -u.y, -u.z, __uint_as_float(0xffffffffu));  // the gap row: no vertices known
+        if (j < rn) f = hand[tpid[t]].d[j];
+        if (cb == kSearchBin) {
+            int type, nv, off;
+            load_meta(s, c, type, nv, off);
+            const f3 d = k ? mk(-f.x, -f.y, -f.z) : mk(f.x, f.y, f.z);
+            for (int h = 0; h < num; ++h) {
+                const int w = warp_hull_argmax(s.verts32, __shfl_sync(kAll, off, h), max(__shfl_sync(kAll, nv, h), 1),
+                                               mk(__shfl_sync(kAll, d.x, h), __shfl_sync(kAll, d.y, h),
+                                                  __shfl_sync(kAll, d.z, h)));
+                if (ln == h) vi = w;
+            }
+        } else {
+            vi = handoff_vertex(f, k);
+        }
+        if (on) {
+            // the polytope vertices phase A took along this row's direction are read, not searched again
+            const f3 df = k ? mk(-f.x, -f.y, -f.z) : mk(f.x, f.y, f.z);
+            Col<double> cl;
+            load_col(s, c, cl);
+            const d3 x = RefineSupportT<MESH>::eval_at(cl, s, mk(widen(df.x), widen(df.y), widen(df.z)), df, vi);
+            double* r = rows + t + (6 * j + 3 * k) * BLOCK;
+            r[0] = x.x;
+            r[BLOCK] = x.y;
+            r[2 * BLOCK] = x.z;
+        }
+        __syncwarp();
+    }
+    __syncthreads();
     // class of the checks: 0 touching (four rows), 1-3 separated with that many rows, 4 none
     const int cls = touch ? 0 : (sep ? nr : 4);
-    if (cls == 4 && slot < cap) {
+    if (cls == 4 && in) {
         // a pair R does not check goes to B as it is (rows of a pair of another shape are kept), or
         // is not R's at all
         if (mine) {
@@ -333,8 +434,6 @@ __global__ void __launch_bounds__(BLOCK) k_gjk_mixed_r(d3d_store s, const int32_
         lists.run_flag[slot] = (int8_t)mine;
         lists.run_pid[slot] = pid;
     }
-    tv[threadIdx.x] = v;
-    tpid[threadIdx.x] = pid;
     tita[threadIdx.x] = it_a;
     tcls[threadIdx.x] = cls | (nr << 8);
     int rank = 0;
@@ -360,8 +459,8 @@ __global__ void __launch_bounds__(BLOCK) k_gjk_mixed_r(d3d_store s, const int32_
         const int owner = tperm[threadIdx.x];
         const int x = tcls[owner];
         const int c = x & 0xff, rn = x >> 8;
-        r_finish<BLOCK>(rows + owner, rn, c >= 1, c == 0, tv[owner], tita[owner], tpid[owner],
-                        (int64_t)blockIdx.x * BLOCK + owner, opt, o, lists);
+        r_finish<BLOCK>(rows + owner, rn, c >= 1, c == 0, tv[owner], tita[owner], tpid[owner], slot0 + owner, opt, o,
+                        lists);
     }
 }
 
@@ -372,6 +471,9 @@ __global__ void __launch_bounds__(BLOCK) k_gjk_mixed_b(d3d_store s, const int32_
                                                         const Handoff* __restrict__ hand, DistanceOut o, Lists lists) {
     __shared__ double rows[24 * BLOCK];
     const int64_t n = (int64_t)lists.ctr[kNumRun];
+    // a short list is spread over the grid's warps: its lanes would run their pairs' different
+    // paths one after the other
+    if ((int)(threadIdx.x & 31) >= spread_lanes(n, BLOCK)) return;
     const JoltEps<double> E = reference_eps<double>();
     const double tol_sq = opt.tolerance * opt.tolerance;
     PhaseB<SmemRows<double, BLOCK>> B;
@@ -450,7 +552,10 @@ __global__ void __launch_bounds__(BLOCK) k_gjk_mixed_b(d3d_store s, const int32_
 __global__ void __launch_bounds__(128) k_gjk_mixed_end(d3d_gjk_options opt, DistanceOut o, Lists lists) {
     const int64_t n = (int64_t)lists.ctr[kNumEnd];
     const JoltEps<double> E = reference_eps<double>();
-    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t lanes = spread_lanes(n, 128), warps = (int64_t)gridDim.x * 4;  // as in B
+    const int ln = threadIdx.x & 31;
+    if (ln >= lanes) return;
+    for (int64_t k = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * lanes + ln; k < n; k += warps * lanes) {
         const int32_t pid = lists.ends[k];
         const EndRecord& e = lists.records[pid];
         GjkLoop<double, RegRows<double>> g;
@@ -515,13 +620,25 @@ int launch_mixed(const d3d_store& store, const int32_t* i1, const int32_t* i2, c
                  const Lists& lists, void* select_temp, size_t select_bytes, int per_sm, cudaStream_t stream) {
     const float tol_sq = (float)(opt.tolerance * opt.tolerance);
     const void* ka = (const void*)k_gjk_mixed_a<BLOCK, MESH>;
-    k_gjk_mixed_a<BLOCK, MESH><<<persistent_blocks(ka, BLOCK, n, per_sm), BLOCK, 0, stream>>>(
-        store, i1, i2, order, n, n_dev, tol_sq, (float)opt.max_distance_squared, opt.max_iterations, hand, o,
-        lists);
+    const int full = persistent_blocks(ka, BLOCK, 32 * n, per_sm);  // every block the GPU holds, down to a pair per warp
+    if (n >= (int64_t)full * BLOCK)
+        k_gjk_mixed_a<BLOCK, MESH><<<full, BLOCK, 0, stream>>>(store, i1, i2, order, n, n_dev, tol_sq,
+                                                               (float)opt.max_distance_squared, opt.max_iterations,
+                                                               hand, o, lists);
+    else
+        k_gjk_mixed_a_spread<BLOCK, MESH><<<full, BLOCK, 0, stream>>>(
+            store, i1, i2, order, n, n_dev, tol_sq, (float)opt.max_distance_squared, opt.max_iterations, hand, o,
+            lists);
     int rc = check_launch("d3d_gjk_distance (mixed, FP32 phase)");
     if (rc) return rc;
-    k_gjk_mixed_r<kRefineBlock, MESH><<<grid_for(n, kRefineBlock), kRefineBlock, 0, stream>>>(
-        store, i1, i2, order, n, n_dev, opt, hand, o, lists);
+    // fewer slots per block where full blocks would leave SMs idle
+    int sms = 1, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int64_t per = (n + 2 * sms - 1) / (2 * sms);
+    per = per < 16 ? 16 : (per > kRefineBlock ? kRefineBlock : per);
+    k_gjk_mixed_r<kRefineBlock, MESH><<<grid_for(n, (int)per), kRefineBlock, 0, stream>>>(
+        store, i1, i2, order, n, (int)per, n_dev, opt, hand, o, lists);
     rc = check_launch("d3d_gjk_distance (mixed, refinement pass)");
     if (rc) return rc;
     // the flagged pairs, in the order of the slots
@@ -532,11 +649,11 @@ int launch_mixed(const d3d_store& store, const int32_t* i1, const int32_t* i2, c
         return D3D_ERR_CUDA;
     }
     const void* kb = (const void*)k_gjk_mixed_b<BLOCK, MESH>;
-    k_gjk_mixed_b<BLOCK, MESH><<<persistent_blocks(kb, BLOCK, n, per_sm), BLOCK, 0, stream>>>(store, i1, i2, opt,
+    k_gjk_mixed_b<BLOCK, MESH><<<persistent_blocks(kb, BLOCK, 32 * n, per_sm), BLOCK, 0, stream>>>(store, i1, i2, opt,
                                                                                              hand, o, lists);
     rc = check_launch("d3d_gjk_distance (mixed, FP64 loop)");
     if (rc) return rc;
-    k_gjk_mixed_end<<<persistent_blocks((const void*)k_gjk_mixed_end, 128, n), 128, 0, stream>>>(opt, o, lists);
+    k_gjk_mixed_end<<<persistent_blocks((const void*)k_gjk_mixed_end, 128, 32 * n), 128, 0, stream>>>(opt, o, lists);
     return check_launch("d3d_gjk_distance (mixed, end pass)");
 }
 

@@ -4,6 +4,7 @@
 #pragma once
 
 #include "jolt.cuh"
+#include "typelist.cuh"
 
 namespace d3d {
 
@@ -103,7 +104,8 @@ __device__ __forceinline__ int box_corner(const float* R, f3 d) {
 // the MeshGraph branch, for kernels launched on stores without meshes.  A
 // non-null `vi` receives the vertex a box, hull or MeshGraph support took
 // (unchanged for the other types), so that the FP64 phases can take the same
-// vertex without searching again (RefineSupportT::eval_at).
+// vertex without searching again (RefineSupportT::eval_at); a hull's vertex
+// that is known already comes in *vi (>= 0).
 template <bool MESH>
 struct FastSupportT {
     static __device__ __forceinline__ f3 base(const Col<float>& c, const d3d_store& s, f3 d, int* vi = nullptr) {
@@ -114,13 +116,20 @@ struct FastSupportT {
         }
         if (c.type == D3D_BOX || c.type == D3D_HULL) {
             if (c.nv < 1) return mk(NAN, NAN, NAN);
-            const int k = hull_argmax(s.verts32, c.off, c.nv, d);
+            const int k = vi && *vi >= 0 ? *vi : hull_argmax(s.verts32, c.off, c.nv, d);
             if (vi) *vi = k;
             return load_vertex(s.verts32, c.off + k);
         }
         if (c.type == D3D_SPHERE) {
             const float n2 = dot(d, d);
             const f3 ctr = mk(c.t[0], c.t[1], c.t[2]);
+            if (vi) {
+                // phase A's roundings, the same in both of its kernels: x and y fused, z not (left to the
+                // compiler they depend on the code around)
+                const float f = c.p[0] * rsqrtf(n2);
+                return n2 == 0.f ? ctr + mk(0.f, 0.f, c.p[0])
+                                 : mk(fmaf(d.x, f, ctr.x), fmaf(d.y, f, ctr.y), __fadd_rn(ctr.z, __fmul_rn(d.z, f)));
+            }
             return n2 == 0.f ? ctr + mk(0.f, 0.f, c.p[0]) : ctr + d * (c.p[0] * rsqrtf(n2));
         }
         if (MESH && c.type == D3D_MESH) {
@@ -142,29 +151,33 @@ using FastSupport = FastSupportT<true>;
 template <bool MESH>
 struct RefineSupportT {
     static __device__ __forceinline__ d3 eval(const Col<double>& c, const d3d_store& s, d3 d) {
-        return margin_fast(s, c, base(c, s, d), d);
+        return margin_fast(s, c, base(c, s, d, rounded(d)), d);
+    }
+    static __device__ __forceinline__ f3 rounded(d3 d) {
+        return mk(__double2float_rn(d.x), __double2float_rn(d.y), __double2float_rn(d.z));
     }
 
-    // eval, given the vertex FastSupport took along the FP32 rounding of d
-    // (vi >= 0; -1: unknown): a box, hull or MeshGraph reads that vertex
-    // instead of searching again (the same search on the same FP32 inputs
-    // would return it), the other types evaluate as eval does.
-    static __device__ __forceinline__ d3 eval_at(const Col<double>& c, const d3d_store& s, d3 d, int vi) {
+    // eval, given the FP32 rounding df of d and the vertex FastSupport took
+    // along it (vi >= 0; -1: unknown): a box, hull or MeshGraph reads that
+    // vertex instead of searching again (the same search on the same FP32
+    // inputs would return it), the other types evaluate as eval does.
+    static __device__ __forceinline__ d3 eval_at(const Col<double>& c, const d3d_store& s, d3 d, f3 df, int vi) {
         if (vi >= 0 && vi < c.nv) {
             if (c.type == D3D_BOX || c.type == D3D_HULL) return margin_fast(s, c, load_vertex(s.verts64, c.off + vi), d);
             if (MESH && c.type == D3D_MESH)
                 return margin_fast(s, c, xform(c.R, c.t, load_vertex(s.verts64, c.off + vi)), d);
         }
-        return eval(c, s, d);
+        return margin_fast(s, c, base(c, s, d, df), d);
     }
 
-    static __device__ __forceinline__ d3 base(const Col<double>& c, const d3d_store& s, d3 d) {
-        const f3 df = mk(__double2float_rn(d.x), __double2float_rn(d.y), __double2float_rn(d.z));
+    // The FP32 record (FastSupport's view) is read where a discrete choice needs it: rounding the
+    // FP64 one again costs an FP64-pipe instruction per value.
+    static __device__ __forceinline__ d3 base(const Col<double>& c, const d3d_store& s, d3 d, f3 df) {
+        const float* rec = s.rec32 + (size_t)c.idx * 16;
         if (c.type == D3D_BOX && c.nv == 8) {
-            // the FP32 record's rotation, as FastSupport sees it
             float Rf[9];
 #pragma unroll
-            for (int k = 0; k < 9; ++k) Rf[k] = __double2float_rn(c.R[k]);
+            for (int k = 0; k < 9; ++k) Rf[k] = __ldg(rec + k);
             return load_vertex(s.verts64, c.off + box_corner(Rf, df));
         }
         if (c.type == D3D_BOX || c.type == D3D_HULL) {
@@ -183,29 +196,40 @@ struct RefineSupportT {
             cf.nv = c.nv;
             cf.off = c.off;
             cf.idx = c.idx;
-            for (int k = 0; k < 9; ++k) cf.R[k] = __double2float_rn(c.R[k]);
+            for (int k = 0; k < 9; ++k) cf.R[k] = __ldg(rec + k);
             return xform(c.R, c.t, load_vertex(s.verts64, c.off + mesh_climb<true>(cf, s, rt_mul(cf.R, df))));
         }
         bool up = false;
         if (c.type == D3D_CAPSULE || c.type == D3D_CYLINDER || c.type == D3D_CONE) {
-            // the FP32 record's rotation: column 2 (capsule, cylinder) or all (cone)
+            // the rotation's column 2 (capsule, cylinder) or all of it (cone)
             float Rf[9] = {};
-            Rf[2] = __double2float_rn(c.R[2]);
-            Rf[5] = __double2float_rn(c.R[5]);
-            Rf[8] = __double2float_rn(c.R[8]);
+            Rf[2] = __ldg(rec + 2);
+            Rf[5] = __ldg(rec + 5);
+            Rf[8] = __ldg(rec + 8);
             if (c.type == D3D_CONE) {
-                Rf[0] = __double2float_rn(c.R[0]);
-                Rf[1] = __double2float_rn(c.R[1]);
-                Rf[3] = __double2float_rn(c.R[3]);
-                Rf[4] = __double2float_rn(c.R[4]);
-                Rf[6] = __double2float_rn(c.R[6]);
-                Rf[7] = __double2float_rn(c.R[7]);
+                Rf[0] = __ldg(rec + 0);
+                Rf[1] = __ldg(rec + 1);
+                Rf[3] = __ldg(rec + 3);
+                Rf[4] = __ldg(rec + 4);
+                Rf[6] = __ldg(rec + 6);
+                Rf[7] = __ldg(rec + 7);
             }
-            up = upper_feature(c.type, Rf, __double2float_rn(c.p[0]), __double2float_rn(c.p[1]), df);
+            up = upper_feature(c.type, Rf, __ldg(rec + 12), __ldg(rec + 13), df);
         }
         return xform(c.R, c.t, local_point(c, rt_mul(c.R, d), up));
     }
 };
+
+// The double of a float, by its bits (a conversion instruction runs on the
+// FP64 pipe); zeros, infinities, NaNs and denormals take the conversion.
+__device__ __forceinline__ double widen(float x) {
+    const unsigned u = __float_as_uint(x);
+    if ((u & 0x7f800000u) - 0x00800000u < 0x7f000000u) {
+        const unsigned hi = (u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20));
+        return __hiloint2double((int)hi, (int)(u << 29));
+    }
+    return (u << 1) == 0u ? __hiloint2double((int)u, 0) : (double)x;
+}
 
 using RefineSupport = RefineSupportT<true>;
 
@@ -287,14 +311,27 @@ __device__ __forceinline__ void pa_begin(PhaseALoop<Rows>& L) {
     L.it = 0;
 }
 
-// one iteration; -1 while running, else a PhaseAOutcome
-template <bool MESH, typename Rows>
-__device__ __forceinline__ int pa_step(PhaseALoop<Rows>& L, const d3d_store& s, int a, int b, float tol_sq, float max_d2,
-                                       int max_iter) {
+// Hulls of at least kShareMin vertices on at most kShareMax lanes are scanned
+// by the whole warp, one after the other, instead of by their lanes alone: a
+// lane takes ~35 cycles per vertex (a load and a dependent compare), the warp
+// ~250 per hull and 45 per 32 vertices.
+constexpr int kShareMin = 24;
+constexpr int kShareMax = 6;
+
+// One iteration; -1 while running (or off), else a PhaseAOutcome.  SHARE: all
+// 32 lanes call it together, `on` marks those with a pair, and hulls are
+// shared as above; otherwise the lanes that call it all have a pair.
+template <bool MESH, bool SHARE, typename Rows>
+__device__ __forceinline__ int pa_step(PhaseALoop<Rows>& L, bool on, const d3d_store& s, int a, int b, float tol_sq,
+                                       float max_d2, int max_iter) {
+    constexpr unsigned kAll = 0xffffffffu;
     const JoltEps<float> E = fp32_eps();
-    if (L.it >= max_iter) return PA_FAILED;
-    ++L.it;
-    const unsigned together = __activemask();
+    if (!SHARE) {
+        if (L.it >= max_iter) return PA_FAILED;
+        ++L.it;
+    }
+    const bool go = !SHARE || (on && L.it < max_iter);
+    const unsigned together = SHARE ? kAll : __activemask();
     f3 p, q;
     // the vertices the polytope supports took, 16 bits per collider (0xffff: none), ride in the
     // Q row of the simplex (phase A reads only Y and the directions in P) to the handoff
@@ -302,18 +339,41 @@ __device__ __forceinline__ int pa_step(PhaseALoop<Rows>& L, const d3d_store& s, 
 #pragma unroll 1
     for (int k = 0; k < 2; ++k) {
         Col<float> c;
-        load_col(s, k ? b : a, c);
+        c.type = -1;
+        if (go) load_col(s, k ? b : a, c);
         int vi = -1;
-        const f3 x = FastSupportT<MESH>::eval(c, s, k ? -L.dir : L.dir, &vi);
-        vis |= (unsigned)(vi >= 0 && vi < 0xffff ? vi : 0xffff) << (16 * k);
-        if (k)
-            q = x;
-        else
-            p = x;
+        if (SHARE) {
+            const f3 d = k ? -L.dir : L.dir;
+            unsigned shared = __ballot_sync(kAll, go && c.type == D3D_HULL && c.nv >= kShareMin);
+            if (shared && __popc(shared) <= kShareMax) {
+                while (shared) {
+                    const int owner = __ffs(shared) - 1;
+                    shared &= shared - 1;
+                    const int w =
+                        warp_hull_argmax(s.verts32, __shfl_sync(kAll, c.off, owner), __shfl_sync(kAll, c.nv, owner),
+                                         mk(__shfl_sync(kAll, d.x, owner), __shfl_sync(kAll, d.y, owner),
+                                            __shfl_sync(kAll, d.z, owner)));
+                    if ((int)(threadIdx.x & 31) == owner) vi = w;
+                }
+            }
+        }
+        if (go) {
+            const f3 x = FastSupportT<MESH>::eval(c, s, k ? -L.dir : L.dir, &vi);
+            vis |= (unsigned)(vi >= 0 && vi < 0xffff ? vi : 0xffff) << (16 * k);
+            if (k)
+                q = x;
+            else
+                p = x;
+        }
     }
     // reconverge after the type- and size-dependent supports, so that the
     // lanes solve their simplices together (see gjk_step)
     __syncwarp(together);
+    if (SHARE) {
+        if (!on) return -1;
+        if (!go) return PA_FAILED;
+        ++L.it;
+    }
     f3 w = p - q;
     float dd = dot(L.dir, w);
     if (dd < 0.f && dd * dd > L.vl * max_d2) return PA_CLIPPED;
