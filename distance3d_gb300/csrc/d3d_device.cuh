@@ -67,6 +67,8 @@ struct Compare {
     static __device__ __forceinline__ bool below0(T x) { return x < T(0); }
     static __device__ __forceinline__ bool not_below0(T x) { return x >= T(0); }
     static __device__ __forceinline__ bool not_above0(T x) { return x <= T(0); }
+    static __device__ __forceinline__ bool lt_sq(T a, T b) { return a < b; }
+    static __device__ __forceinline__ bool le_sq(T a, T b) { return a <= b; }
 };
 #ifndef D3D_FP_COMPARES
 template <>
@@ -98,6 +100,13 @@ struct Compare<double> {
     static __device__ __forceinline__ bool not_above0(double x) {
         return bits(x) - 0x8000000000000000ull <= (unsigned long long)kInf || bits(x) == 0ull;
     }
+    // operands that are +0 or above, or NaN (without a sign): squared lengths
+    static __device__ __forceinline__ bool lt_sq(double a, double b) {
+        return bits(a) < bits(b) && bits(b) <= (unsigned long long)kInf;
+    }
+    static __device__ __forceinline__ bool le_sq(double a, double b) {
+        return bits(a) <= bits(b) && bits(b) <= (unsigned long long)kInf;
+    }
 };
 #endif
 template <typename T>
@@ -112,6 +121,11 @@ template <typename T>
 __device__ __forceinline__ bool not_below0(T x) { return Compare<T>::not_below0(x); }
 template <typename T>
 __device__ __forceinline__ bool not_above0(T x) { return Compare<T>::not_above0(x); }
+// a < b, a <= b of values that are +0, above, or NaN
+template <typename T>
+__device__ __forceinline__ bool lt_sq(T a, T b) { return Compare<T>::lt_sq(a, b); }
+template <typename T>
+__device__ __forceinline__ bool le_sq(T a, T b) { return Compare<T>::le_sq(a, b); }
 
 // np.dot of two 3-vectors (ddot), np.linalg.norm, and the small GEMMs of
 // geometry.py:157 / containment.py:147: fma(a2,b2, fma(a1,b1, a0*b0))
@@ -289,13 +303,15 @@ __device__ __forceinline__ Filter32 filter32(V3<double> d) {
     f.dabs = fabsf(f.dx) + fabsf(f.dy) + fabsf(f.dz);
     return f;
 }
-// (s_k, E_k) of vertex row `row` of the FP32 mirror
-__device__ __forceinline__ float2 filter_product(const float* v32, int row, const Filter32& f) {
-    const float4 v = __ldg(reinterpret_cast<const float4*>(v32) + row);
+// (s_k, E_k) of vertex v of the FP32 mirror
+__device__ __forceinline__ float2 filter_product(float4 v, const Filter32& f) {
     const float s = fmaf(v.z, f.dz, fmaf(v.x, f.dx, v.y * f.dy));
     const float sa = fmaf(fabsf(v.z), fabsf(f.dz), fmaf(fabsf(v.x), fabsf(f.dx), fabsf(v.y) * fabsf(f.dy)));
     const float e = fmaf(sa, 0x1p-20f, 0x1p-126f * (fabsf(v.x) + fabsf(v.y) + fabsf(v.z) + f.dabs + 1.f));
     return make_float2(s, e);
+}
+__device__ __forceinline__ float2 filter_product(const float* v32, int row, const Filter32& f) {
+    return filter_product(__ldg(reinterpret_cast<const float4*>(v32) + row), f);
 }
 
 __device__ __forceinline__ int hull_argmax_filtered(const double* v64, const float* v32, int off, int nv, V3<double> d) {

@@ -139,18 +139,28 @@ __device__ __forceinline__ int warp_argmax(const d3d_store& st, int off, int nv,
     float lo = -INFINITY, top = -INFINITY, second = -INFINITY;
     int ti = 0;
     bool fin = isfinite(f.dabs);
-#pragma unroll 2
-    for (int k = ln; k < nv; k += 32) {
-        const float2 se = filter_product(st.verts32, off + k, f);
-        fin &= isfinite(se.x) && isfinite(se.y);
-        lo = fmaxf(lo, se.x - se.y);
-        const float up = se.x + se.y;
-        if (up > top) {
-            second = top;
-            top = up;
-            ti = k;
-        } else {
-            second = fmaxf(second, up);
+    // the loads of four rounds together
+    const float4* const v = reinterpret_cast<const float4*>(st.verts32) + off;
+#pragma unroll 1
+    for (int k0 = ln; k0 < nv; k0 += 128) {
+        float4 x[4];
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+            if (k0 + 32 * h < nv) x[h] = __ldg(v + k0 + 32 * h);
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            if (k0 + 32 * h >= nv) continue;
+            const float2 se = filter_product(x[h], f);
+            fin &= isfinite(se.x) && isfinite(se.y);
+            lo = fmaxf(lo, se.x - se.y);
+            const float up = se.x + se.y;
+            if (up > top) {
+                second = top;
+                top = up;
+                ti = k0 + 32 * h;
+            } else {
+                second = fmaxf(second, up);
+            }
         }
     }
     const bool finite = __all_sync(kAll, fin);
@@ -223,11 +233,11 @@ __device__ __forceinline__ void hull_supports(Mem<S, PQ>& m, const d3d_store& st
 }
 
 // gjk_step_end (distance) or the rest of gjk_intersection_loop's iteration,
-// for slot s and the result of its solve.  `hit`: the intersection form's
-// outcome, -1 while it runs.
-template <int S, int PQ>
+// for slot s and the result of its solve; ysq(r) is |Y|^2 of place r.  Returns
+// the intersection form's outcome, -1 while it runs.
+template <int S, int PQ, typename Ysq>
 __device__ __forceinline__ int finish_step(Mem<S, PQ>& m, int s, bool closer, d3 nv, double nl, int set, double tol_sq,
-                                           int max_iter, const JoltEps<double>& E) {
+                                           int max_iter, const JoltEps<double>& E, Ysq ysq) {
     constexpr bool kDistance = PQ == 4;
     unsigned mt = m.meta[s];
     unsigned perm = mt & 0xffu;
@@ -244,20 +254,19 @@ __device__ __forceinline__ int finish_step(Mem<S, PQ>& m, int s, bool closer, d3
         dir = mk(m.dir[s], m.dir[S + s], m.dir[2 * S + s]);
         vl = m.vl[s];
     }
-    if (!kDistance && (set == 15 || le(vl, tol_sq))) return 1;
+    if (!kDistance && (set == 15 || le_sq(vl, tol_sq))) return 1;
     int ending = -1;  // GjkEnd
     if (set == 15) {
         ending = GJK_INTERSECTION;
     } else {
         if (!kDistance) {
             // max |Y|^2 over the rows before compaction
-            double y = dot(m.y(mt, 0, s), m.y(mt, 0, s));
+            double y = ysq(place_of(mt, 0));
             for (int r = 1; r < n; ++r) {
-                const d3 v = m.y(mt, r, s);
-                const double l = dot(v, v);
-                if (lt(y, l)) y = l;
+                const double l = ysq(place_of(mt, r));
+                if (lt_sq(y, l)) y = l;
             }
-            if (le(vl, E.isect * y)) return 1;
+            if (le_sq(vl, E.isect * y)) return 1;
             dir = -dir;
             const double prev = m.prev[s];
             if (le(prev - vl, E.conv * prev)) return 0;
@@ -274,15 +283,14 @@ __device__ __forceinline__ int finish_step(Mem<S, PQ>& m, int s, bool closer, d3
         perm = np;
         n = k;
         if (kDistance) {
-            bool touch = le(vl, tol_sq);
+            bool touch = le_sq(vl, tol_sq);
             if (!touch) {
-                double y = dot(m.row(m.Y, perm & 3, s), m.row(m.Y, perm & 3, s));
+                double y = ysq(place_of(perm, 0));
                 for (int r = 1; r < n; ++r) {
-                    const d3 v = m.row(m.Y, (perm >> (2 * r)) & 3, s);
-                    const double l = dot(v, v);
-                    if (lt(y, l)) y = l;
+                    const double l = ysq(place_of(perm, r));
+                    if (lt_sq(y, l)) y = l;
                 }
-                touch = le(vl, E.isect * y);
+                touch = le_sq(vl, E.isect * y);
             }
             if (touch) {
                 ending = GJK_INTERSECTION;
@@ -313,6 +321,15 @@ __device__ __forceinline__ int finish_step(Mem<S, PQ>& m, int s, bool closer, d3
     return -1;
 }
 
+template <int S, int PQ>
+__device__ __forceinline__ int finish_step(Mem<S, PQ>& m, int s, bool closer, d3 nv, double nl, int set, double tol_sq,
+                                           int max_iter, const JoltEps<double>& E) {
+    return finish_step(m, s, closer, nv, nl, set, tol_sq, max_iter, E, [&](int r) {
+        const d3 v = m.row(m.Y, r, s);
+        return dot(v, v);
+    });
+}
+
 // The pair of slot s has ended in the intersection form.
 template <int S, int PQ>
 __device__ __forceinline__ void put_hit(Mem<S, PQ>& m, int s, int hit, int8_t* hits, int8_t* status) {
@@ -330,10 +347,10 @@ __device__ __forceinline__ void put_hit(Mem<S, PQ>& m, int s, int hit, int8_t* h
 // after the other: three edges and the face with six divisions in all.
 __device__ __forceinline__ d3 flat_triangle(d3 a, d3 b, d3 c, const JoltEps<double>& E, int& set) {
     const d3 ab = b - a, ac = c - a, bc = c - b;
-    const bool shorter = lt(dot(bc, bc), dot(ac, ac));
+    const bool shorter = lt_sq(dot(bc, bc), dot(ac, ac));
     const d3 n = cross(ab, mk(shorter ? bc.x : ac.x, shorter ? bc.y : ac.y, shorter ? bc.z : ac.z));
     const double nl = dot(n, n);
-    if (lt(nl, E.sq)) return cp_triangle(a, b, c, E, set);  // degenerate
+    if (lt_sq(nl, E.sq)) return cp_triangle(a, b, c, E, set);  // degenerate
     const double d1 = dot(ab, -a), d2 = dot(ac, -a), d3_ = dot(ab, -b), d4 = dot(ac, -b), d5 = dot(ab, -c),
                  d6 = dot(ac, -c);
     const double vc = d1 * d4 - d3_ * d2, vb = d5 * d2 - d1 * d6, va = d3_ * d6 - d5 * d4;
@@ -455,7 +472,7 @@ __device__ __forceinline__ void solve_tetrahedra(Mem<S, PQ>& m, int first, int c
             const double fd = __shfl_sync(kAll, d2, src);
             const d3 fv = mk(__shfl_sync(kAll, r.x, src), __shfl_sync(kAll, r.y, src), __shfl_sync(kAll, r.z, src));
             const int fs = __shfl_sync(kAll, set, src);
-            if (mine && (f == 0 || lt(fd, bd))) {
+            if (mine && (f == 0 || lt_sq(fd, bd))) {
                 bd = bl = fd;
                 bv = fv;
                 bs = fs;
@@ -464,9 +481,142 @@ __device__ __forceinline__ void solve_tetrahedra(Mem<S, PQ>& m, int first, int c
     }
     if (ln < count) {
         const int s = m.solve[first + ln];
-        put_hit(m, s, finish_step(m, s, lt(bl, m.prev[s]), bv, bl, bs, tol_sq, max_iter, E), hits, status);
+        put_hit(m, s, finish_step(m, s, lt_sq(bl, m.prev[s]), bv, bl, bs, tol_sq, max_iter, E), hits, status);
     }
     __syncwarp();  // the task list is rewritten by the warp's next chunk
+}
+
+__device__ __forceinline__ double shfl8(double x, int j) { return __shfl_sync(kAll, x, j, 8); }
+__device__ __forceinline__ d3 shfl8(d3 v, int j) { return mk(shfl8(v.x, j), shfl8(v.y, j), shfl8(v.z, j)); }
+__device__ __forceinline__ double coord(d3 v, int j) { return j == 0 ? v.x : (j == 1 ? v.y : v.z); }
+
+// One triangle or tetrahedron by the whole warp, where a block has no more of
+// them than warps: the length of the chain counts then, not the pipe.  Eight
+// lanes take each face of a tetrahedron (a triangle has one), tested by its
+// plane or not, and spread the independent products of flat_triangle: the six
+// corner dots and two edge lengths on a lane each, the normal's and the
+// closest point's components on three, so that a solve is ~45 dependent FP64
+// instructions instead of ~150.  The values are flat_triangle's and
+// outside_planes', operation by operation.  1,000 primitive pairs: 609 -> 505 us.
+template <int S, int PQ>
+__device__ __forceinline__ void solve_wide(Mem<S, PQ>& m, int s, double tol_sq, int max_iter, const JoltEps<double>& E,
+                                           int8_t* hits, int8_t* status) {
+    const int ln = threadIdx.x & 31, f = ln >> 3, j = ln & 7;
+    const unsigned mt = m.meta[s];
+    const bool tetra = meta_n(mt) == 4;
+    const int i0 = f == 3 ? 1 : 0;
+    const int i1 = f == 0 ? 1 : (f == 1 ? 2 : 3);
+    const int i2 = f == 0 ? 2 : (f == 1 ? 3 : (f == 2 ? 1 : 2));
+    const d3 a = m.y(mt, i0, s), b = m.y(mt, i1, s), c = m.y(mt, i2, s);
+    // lanes 0-5: d1 .. d6 (ab or ac against -a, -b, -c), 6: bc . bc, 7: ac . ac
+    const bool toc = j == 1 || j == 3 || j >= 5;
+    const d3 e = (toc ? c : b) - (j == 6 ? b : a);
+    const d3 u = j < 2 ? -a : (j < 4 ? -b : (j < 6 ? -c : e));
+    const double dj = dot(e, u);
+    const double d1 = shfl8(dj, 0), d2 = shfl8(dj, 1), d3_ = shfl8(dj, 2), d4 = shfl8(dj, 3), d5 = shfl8(dj, 4),
+                 d6 = shfl8(dj, 5);
+    const d3 ab = shfl8(e, 0), ac = shfl8(e, 1), bc = shfl8(e, 6);
+    const bool shorter = lt_sq(shfl8(dj, 6), shfl8(dj, 7));
+    const d3 x = shorter ? bc : ac;
+    // lanes 0-2: the normal ab x (bc or ac), 3-5: vc, vb, va
+    double n1 = 0.0, n2 = 0.0, n3 = 0.0, n4 = 0.0;
+    if (j < 3) {
+        const int k = j == 2 ? 0 : j + 1, l = j == 0 ? 2 : j - 1;
+        n1 = coord(ab, k);
+        n2 = coord(x, l);
+        n3 = coord(ab, l);
+        n4 = coord(x, k);
+    } else if (j < 6) {
+        n1 = j == 3 ? d1 : (j == 4 ? d5 : d3_);
+        n2 = j == 3 ? d4 : (j == 4 ? d2 : d6);
+        n3 = j == 3 ? d3_ : (j == 4 ? d1 : d5);
+        n4 = j == 3 ? d2 : (j == 4 ? d6 : d4);
+    }
+    const double pj = n1 * n2 - n3 * n4;
+    const d3 n = mk(shfl8(pj, 0), shfl8(pj, 1), shfl8(pj, 2));
+    const double vc = shfl8(pj, 3), vb = shfl8(pj, 4), va = shfl8(pj, 5);
+    // the plane of the face (tetrahedra): normal ab x ac, and the fourth corner's edge from corner 0
+    d3 cr = n, e3 = n;
+    if (tetra) {
+        const int k = j == 2 ? 0 : j + 1, l = j == 0 ? 2 : j - 1;
+        const double cj = coord(ab, k) * coord(ac, l) - coord(ab, l) * coord(ac, k);
+        const double ej = coord(m.y(mt, f == 0 ? 3 : (f == 2 ? 2 : 1), s), j) - coord(m.y(mt, 0, s), j);
+        cr = mk(shfl8(cj, 0), shfl8(cj, 1), shfl8(cj, 2));
+        e3 = mk(shfl8(ej, 0), shfl8(ej, 1), shfl8(ej, 2));
+    }
+    // lanes 0-2: (a + b) + c, 3: d43 + d56, 5: d1 - d3, 6: d2 - d6
+    const double s1 = j < 3 ? coord(a, j) : (j == 3 ? d4 : (j == 4 ? d5 : (j == 5 ? d1 : d2)));
+    const double s2 = j < 3 ? coord(b, j) : (j == 3 || j == 5 ? -d3_ : -d6);
+    const double sj = s1 + s2;
+    const double d43 = shfl8(sj, 3), d56 = shfl8(sj, 4), e13 = shfl8(sj, 5), e26 = shfl8(sj, 6);
+    const double tj = (j < 3 ? sj : d43) + (j < 3 ? coord(c, j) : d56);
+    const d3 sum = mk(shfl8(tj, 0), shfl8(tj, 1), shfl8(tj, 2));
+    const double e46 = shfl8(tj, 3);
+    // lane 0: |n|^2, 1: (a + b + c) . n, 2: the origin's side of the plane, 3: the fourth corner's
+    const double uj = dot(j == 0 ? n : (j == 1 ? sum : (j == 2 ? a : e3)), j < 2 ? n : cr);
+    const double nl = shfl8(uj, 0), sn = shfl8(uj, 1), sp = shfl8(uj, 2);
+    double sd = shfl8(uj, 3);
+    if (f == 3) sd = -sd;
+    // flat_triangle's region tests, one value per lane: bit i of a mask is d(i + 1)'s, vc's .. va's
+    // sit at bits 3 - 5, d43's and d56's at 3 and 4
+    const int sh = 8 * f;
+    const unsigned dn = __ballot_sync(kAll, not_above0(dj)) >> sh, du = __ballot_sync(kAll, not_below0(dj)) >> sh;
+    const unsigned pn = __ballot_sync(kAll, not_above0(pj)) >> sh, su = __ballot_sync(kAll, not_below0(sj)) >> sh;
+    const unsigned ord = __ballot_sync(kAll, le(j == 0 ? d4 : d5, j == 0 ? d3_ : d6)) >> sh;  // d4 <= d3, d5 <= d6
+    int set = 7;
+    if ((pn & 32u) && (su & 24u) == 24u) set = 6;
+    if ((pn & 16u) && (du & 2u) && (dn & 32u)) set = 5;
+    if ((du & 32u) && (ord & 2u)) set = 4;
+    if ((pn & 8u) && (du & 1u) && (dn & 4u)) set = 3;
+    if ((du & 4u) && (ord & 1u)) set = 2;
+    if ((dn & 3u) == 3u) set = 1;
+    const bool line = set == 3 || set == 5 || set == 6;
+    const double mj = (j < 3 ? coord(n, j) : 3.0) * (j < 3 ? sn : nl);
+    const double den7 = shfl8(mj, 3);
+    double r1 = coord(set == 2 || set == 6 ? b : (set == 4 ? c : a), j);
+    if (line || set == 7) {
+        const double num = set == 7 ? mj : (set == 3 ? d1 : (set == 5 ? d2 : d43));
+        const double den = set == 7 ? den7 : (set == 3 ? e13 : (set == 5 ? e26 : e46));
+        const double q = num / den;
+        r1 = line ? r1 + coord(set == 3 ? ab : (set == 5 ? ac : bc), j) * q : q;
+    }
+    __syncwarp();
+    d3 r = mk(shfl8(r1, 0), shfl8(r1, 1), shfl8(r1, 2));
+    if (lt_sq(nl, E.sq)) r = cp_triangle(a, b, c, E, set);  // degenerate
+    const double l = dot(r, r);
+    set = ((set & 1) << i0) | (((set >> 1) & 1) << i1) | (((set >> 2) & 1) << i2);
+    // the faces that see the origin (a triangle's own)
+    const bool up = (__ballot_sync(kAll, above0(sd)) & 0x01010101u) == 0x01010101u;
+    const bool down = (__ballot_sync(kAll, below0(sd)) & 0x01010101u) == 0x01010101u;
+    const bool out = tetra ? (up ? le(-E.plane, sp) : (down ? le(sp, E.plane) : true)) : f == 0;
+    const unsigned vis = __ballot_sync(kAll, out);
+    // place ln's |Y|^2 for the end of the iteration
+    const d3 yv = m.row(m.Y, ln & 3, s);
+    const double yy = dot(yv, yv);
+    // the first face as it is (a NaN included), a later one if strictly closer: the smallest |r|^2,
+    // then the lowest face
+    const unsigned long long lb = (unsigned long long)__double_as_longlong(l);
+    const bool in = j == 0 && out && (f == 0 || lb < 0x7fefffffffffffffull);
+    const unsigned long long key = f == 0 && lb > 0x7ff0000000000000ull ? 0ull : lb;
+    const unsigned khi = __reduce_min_sync(kAll, in ? (unsigned)(key >> 32) : 0xffffffffu);
+    const unsigned klo = __reduce_min_sync(kAll, in && (unsigned)(key >> 32) == khi ? (unsigned)key : 0xffffffffu);
+    const unsigned win = __ballot_sync(kAll, in && key == (((unsigned long long)khi << 32) | klo));
+    const int from = win ? __ffs(win) - 1 : 0;
+    d3 bv = mk(__shfl_sync(kAll, r.x, from), __shfl_sync(kAll, r.y, from), __shfl_sync(kAll, r.z, from));
+    double bl = __shfl_sync(kAll, l, from);
+    int bs = __shfl_sync(kAll, set, from);
+    if (!win) {
+        bv = mk(0.0, 0.0, 0.0);
+        bl = 0.0;
+        bs = 15;
+    }
+    const double y0 = __shfl_sync(kAll, yy, 0), y1 = __shfl_sync(kAll, yy, 1), y2 = __shfl_sync(kAll, yy, 2),
+                 y3 = __shfl_sync(kAll, yy, 3);
+    if (ln == 0)
+        put_hit(m, s,
+                finish_step(m, s, lt_sq(bl, m.prev[s]), bv, bl, bs, tol_sq, max_iter, E,
+                            [=](int p) { return p == 0 ? y0 : (p == 1 ? y1 : (p == 2 ? y2 : y3)); }),
+                hits, status);
 }
 
 // The FP64 GJK distance (PQ = 4) or intersection test (PQ = 1) of the pairs
@@ -657,13 +807,18 @@ __global__ void __launch_bounds__(S, 512 / S) k_gjk_pool(d3d_store st, const int
         __syncthreads();
         // ---- solve
         const int n4 = m.scnt[par][0], n3 = m.scnt[par][1], n2 = m.scnt[par][2], n1 = m.scnt[par][3];
-        const int c4 = (n4 + kTetraChunk - 1) / kTetraChunk, c3 = (n3 + 31) / 32, c2 = (n2 + 31) / 32,
-                  c1 = (n1 + 31) / 32;
+        const bool wide = n4 + n3 <= S / 32;  // no more than warps: each by a whole warp
+        const int c4 = wide ? n4 + n3 : (n4 + kTetraChunk - 1) / kTetraChunk, c3 = wide ? 0 : (n3 + 31) / 32,
+                  c2 = (n2 + 31) / 32, c1 = (n1 + 31) / 32;
         while (true) {
             int x = 0;
             if (ln == 0) x = atomicAdd(&m.next[par][1], 1);
             x = __shfl_sync(kAll, x, 0);
             if (x >= c4 + c3 + c2 + c1) break;
+            if (x < c4 && wide) {
+                solve_wide(m, m.solve[x < n4 ? x : S + x - n4], tol_sq, opt.max_iterations, E, hits, o.status);
+                continue;
+            }
             if (x < c4) {
                 solve_tetrahedra(m, kTetraChunk * x, min(kTetraChunk, n4 - kTetraChunk * x), tol_sq, opt.max_iterations,
                                  E, hits, o.status);
@@ -682,7 +837,7 @@ __global__ void __launch_bounds__(S, 512 / S) k_gjk_pool(d3d_store st, const int
                 else if (k == 2)
                     r = cp_line(r, m.y(mt, 1, s), E, set);
                 const double l = dot(r, r);
-                put_hit(m, s, finish_step(m, s, lt(l, m.prev[s]), r, l, set, tol_sq, opt.max_iterations, E), hits,
+                put_hit(m, s, finish_step(m, s, lt_sq(l, m.prev[s]), r, l, set, tol_sq, opt.max_iterations, E), hits,
                         o.status);
             }
         }

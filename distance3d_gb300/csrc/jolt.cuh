@@ -44,8 +44,8 @@ template <typename T>
 __device__ __forceinline__ void bary_line(V3<T> a, V3<T> b, const JoltEps<T>& E, T& u, T& v) {
     V3<T> ab = b - a;
     T den = dot(ab, ab);
-    if (lt(den, E.sq)) {
-        if (lt(dot(a, a), dot(b, b))) {
+    if (lt_sq(den, E.sq)) {
+        if (lt_sq(dot(a, a), dot(b, b))) {
             u = T(1);
             v = T(0);
         } else {
@@ -67,11 +67,11 @@ template <typename T, bool SCALED = false>
 __device__ __forceinline__ void bary_plane(V3<T> a, V3<T> b, V3<T> c, const JoltEps<T>& E, T& u, T& v, T& w) {
     V3<T> v0 = b - a, v1 = c - a, v2 = c - b;
     T d00 = dot(v0, v0), d11 = dot(v1, v1), d22 = dot(v2, v2);
-    if (le(d00, d22)) {
+    if (le_sq(d00, d22)) {
         T d01 = dot(v0, v1);
         T den = d00 * d11 - d01 * d01;
         if (lt(abs_t(den), SCALED ? E.plane * (d00 * d11) : E.plane)) {
-            if (lt(d11, d00)) {
+            if (lt_sq(d11, d00)) {
                 bary_line(a, b, E, u, v);
                 w = T(0);
             } else {
@@ -88,7 +88,7 @@ __device__ __forceinline__ void bary_plane(V3<T> a, V3<T> b, V3<T> c, const Jolt
         T d12 = dot(v1, v2);
         T den = d11 * d22 - d12 * d12;
         if (lt(abs_t(den), SCALED ? E.plane * (d11 * d22) : E.plane)) {
-            if (lt(d22, d11)) {
+            if (lt_sq(d22, d11)) {
                 bary_line(a, c, E, u, w);
                 v = T(0);
             } else {
@@ -145,22 +145,22 @@ __device__ __forceinline__ V3<T> cp_line(V3<T> a, V3<T> b, const JoltEps<T>& E, 
 template <typename T, bool FAST = false>
 __device__ __forceinline__ V3<T> cp_triangle(V3<T> a, V3<T> b, V3<T> c, const JoltEps<T>& E, int& set) {
     V3<T> ab = b - a, ac = c - a, bc = c - b;
-    V3<T> n = lt(dot(bc, bc), dot(ac, ac)) ? cross(ab, bc) : cross(ab, ac);
+    V3<T> n = lt_sq(dot(bc, bc), dot(ac, ac)) ? cross(ab, bc) : cross(ab, ac);
     T nl = dot(n, n);
-    if (lt(nl, E.sq)) {
+    if (lt_sq(nl, E.sq)) {
         int s, ns;
         V3<T> cp = cp_line(a, b, E, s);
         T best = dot(cp, cp);
         V3<T> q = cp_line(a, c, E, ns);
         T d2 = dot(q, q);
-        if (lt(d2, best)) {
+        if (lt_sq(d2, best)) {
             cp = q;
             best = d2;
             s = (ns & 1) + ((ns & 2) << 1);
         }
         q = cp_line(b, c, E, ns);
         d2 = dot(q, q);
-        if (lt(d2, best)) {
+        if (lt_sq(d2, best)) {
             cp = q;
             s = ns << 1;
         }
@@ -365,7 +365,7 @@ __device__ __forceinline__ bool closest_to_origin(const Simplex<T, Rows>& S, T p
             int ns;
             const V3<T> q = cp_triangle<T, FAST>(row_of(S.Y, i0), row_of(S.Y, i1), row_of(S.Y, i2), E, ns);
             const T d2 = dot(q, q);
-            if (f == 0 || lt(d2, best)) {
+            if (f == 0 || lt_sq(d2, best)) {
                 best = d2;
                 r = q;
                 s = ((ns & 1) << i0) | (((ns >> 1) & 1) << i1) | (((ns >> 2) & 1) << i2);
@@ -373,7 +373,7 @@ __device__ __forceinline__ bool closest_to_origin(const Simplex<T, Rows>& S, T p
         }
     }
     T l = dot(r, r);
-    if (lt(l, prev)) {
+    if (lt_sq(l, prev)) {
         v = r;
         vl = l;
         set = s;
@@ -390,7 +390,7 @@ __device__ __forceinline__ T max_y_len_sq(const Simplex<T, Rows>& S) {
     for (int i = 1; i < 4; ++i)
         if (i < S.n) {
             T l = dot(S.Y[i], S.Y[i]);
-            if (lt(m, l)) m = l;
+            if (lt_sq(m, l)) m = l;
         }
     return m;
 }
@@ -574,7 +574,7 @@ __device__ __forceinline__ bool gjk_step_end(GjkLoop<T, Rows>& g, T tol_sq, cons
         return true;
     }
     simplex_compact<T, true>(g.S, set);
-    if (le(g.vl, tol_sq) || le(g.vl, E.isect * max_y_len_sq(g.S))) {
+    if (le_sq(g.vl, tol_sq) || le_sq(g.vl, E.isect * max_y_len_sq(g.S))) {
         g.vl = T(0);
         g.state = GJK_INTERSECTION;
         return true;
