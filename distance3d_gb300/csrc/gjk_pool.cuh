@@ -103,6 +103,11 @@ struct Mem {
         a[(3 * r + 2) * S + s] = v.z;
     }
     __device__ d3 y(unsigned m, int row_, int s) const { return row(Y, place_of(m, row_), s); }
+    __device__ d3 direction(int s) const { return mk(dir[s], dir[S + s], dir[2 * S + s]); }
+    // the support point of side `side` along the pair's direction
+    __device__ void put_support(int s, int side, d3 x) {
+        put(side ? Q : P, PQ == 4 ? meta_fresh(meta[s]) : 0, s, x);
+    }
 };
 
 // P and Q rows of a pair for closest_points
@@ -191,24 +196,18 @@ __device__ __forceinline__ int warp_argmax(const d3d_store& st, int off, int nv,
     return (__any_sync(kAll, nan0) || i >= (unsigned)nv) ? 0 : (int)i;
 }
 
-// The support of one listed side: base collider type, direction and collider.
-template <int S, int PQ>
-__device__ __forceinline__ void put_support(Mem<S, PQ>& m, int slot, int side, d3 x) {
-    const int r = PQ == 4 ? meta_fresh(m.meta[slot]) : 0;
-    m.put(side ? m.Q : m.P, r, slot, x);
-}
-
-// Up to kHullChunk hulls (list entries e0, e0 + 1, ...), the whole warp on
-// one at a time.
-template <int S, int PQ>
-__device__ __forceinline__ void hull_supports(Mem<S, PQ>& m, const d3d_store& st, int first, int count) {
+// Up to kHullChunk listed hulls (m.list[first ...]: slot << 1 | side), the
+// whole warp on one at a time.  The pool m gives `list`, the colliders
+// col[side S + slot], direction(slot) and put_support(slot, side, point).
+template <int S, typename M>
+__device__ __forceinline__ void hull_supports(M& m, const d3d_store& st, int first, int count) {
     const int ln = threadIdx.x & 31;
     const int e = m.list[first + (ln < count ? ln : count - 1)];
     const int slot = e >> 1, side = e & 1;
     const int ci = m.col[side * S + slot];
     int type, nv, off;
     load_meta(st, ci, type, nv, off);
-    d3 d = mk(m.dir[slot], m.dir[S + slot], m.dir[2 * S + slot]);
+    d3 d = m.direction(slot);
     if (side) d = -d;
     const Filter32 f = filter32(d);
     int win = 0;
@@ -228,8 +227,19 @@ __device__ __forceinline__ void hull_supports(Mem<S, PQ>& m, const d3d_store& st
         Col<double> c;
         load_meta(st, ci, c);
         c.m = c.wrapped ? __ldg(st.rec64 + (size_t)ci * 16 + 15) : 0.0;
-        put_support(m, slot, side, add_margin(c, x, d));
+        m.put_support(slot, side, add_margin(c, x, d));
     }
+}
+
+// The listed support e (slot << 1 | side) of any type but a hull, by one lane.
+template <int S, typename M>
+__device__ __forceinline__ void lane_support(M& m, const d3d_store& st, int e) {
+    const int s = e >> 1, side = e & 1;
+    Col<double> c;
+    load_col(st, m.col[side * S + s], c);
+    d3 d = m.direction(s);
+    if (side) d = -d;
+    m.put_support(s, side, support(c, st, d));
 }
 
 // gjk_step_end (distance) or the rest of gjk_intersection_loop's iteration,
@@ -734,10 +744,10 @@ __global__ void __launch_bounds__(S, 512 / S) k_gjk_pool(d3d_store st, const int
             const int first = __shfl_sync(kAll, task0, bin) + k0;
             const int count = min(csize, cbin - k0);
             if ((bin >> 1) == D3D_HULL) {
-                hull_supports(m, st, first, count);
+                hull_supports<S>(m, st, first, count);
             } else if (ln < count) {
                 const int e = m.list[first + ln];
-                const int s = e >> 1, side = e & 1;
+                const int s = e >> 1;
                 if (bin == kEndBin) {
                     if (kDistance) {
                         const unsigned mt = m.meta[s];
@@ -759,11 +769,7 @@ __global__ void __launch_bounds__(S, 512 / S) k_gjk_pool(d3d_store st, const int
                         m.meta[s] = 0;
                     }
                 } else {
-                    Col<double> cl;
-                    load_col(st, m.col[side * S + s], cl);
-                    d3 d = mk(m.dir[s], m.dir[S + s], m.dir[2 * S + s]);
-                    if (side) d = -d;
-                    put_support(m, s, side, support(cl, st, d));
+                    lane_support<S>(m, st, e);
                 }
             }
             __syncwarp();

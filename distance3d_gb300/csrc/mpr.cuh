@@ -108,9 +108,9 @@ __device__ __forceinline__ bool reach_tolerance(const P& Pt, V3<T> v4, V3<T> d, 
     for (int r = 1; r < 4; ++r) {
         const V3<T> v = Pt.v(r);
         const T e = s4 - dot102(v.x, v.y, v.z, d.x, d.y, d.z);
-        if (r == 1 || e < m) m = e;
+        if (r == 1 || lt(e, m)) m = e;
     }
-    return m < T(tol + kEps);
+    return lt(m, T(tol + kEps));
 }
 
 // :302-317
@@ -119,10 +119,10 @@ __device__ __forceinline__ void expand(const P& Pt, V3<T> pa, V3<T> pb, V3<T> d)
     const V3<T> v4 = pa - pb;
     const V3<T> c = cross(v4, Pt.v(0));
     int r;
-    if (dot(Pt.v(1), c) > T(0))
-        r = dot(Pt.v(2), c) > T(0) ? 1 : 3;
+    if (above0(dot(Pt.v(1), c)))
+        r = above0(dot(Pt.v(2), c)) ? 1 : 3;
     else
-        r = dot(Pt.v(3), c) > T(0) ? 2 : 1;
+        r = above0(dot(Pt.v(3), c)) ? 2 : 1;
     Pt.set(r, pa, pb, d);
 }
 
@@ -166,7 +166,7 @@ __device__ __forceinline__ void begin(const P& Pt, Lane<T>& L, V3<T> c1, V3<T> c
 template <typename T, typename P>
 __device__ __forceinline__ bool enter_refine(const P& Pt, Lane<T>& L) {
     L.d = portal_direction(Pt);
-    if (dot(Pt.v(1), L.d) > T(-10.0 * kEps)) return true;
+    if (lt(T(-10.0 * kEps), dot(Pt.v(1), L.d))) return true;
     L.phase = kRefine;
     L.it = 0;
     return false;
@@ -185,9 +185,9 @@ __device__ int round(const P& Pt, Lane<T>& L, V3<T> pa, V3<T> pb, const d3d_mpr_
     case kV1: {  // :177-201
         Pt.set(1, pa, pb, L.d);
         const V3<T> v1 = Pt.v(1);
-        if (!all_zero(v1) && dot(v1, L.d) < eps) return kMiss;
+        if (!all_zero(v1) && lt(dot(v1, L.d), eps)) return kMiss;
         const V3<T> d = cross(v0, v1);
-        if (dot(d, d) < collinear_eps(v0, v1)) return all_zero(v1) ? kHitV1 : kHitSegment;
+        if (lt_sq(dot(d, d), collinear_eps(v0, v1))) return all_zero(v1) ? kHitV1 : kHitSegment;
         L.d = norm_vector(d);
         L.phase = kV2;
         return kRunning;
@@ -195,9 +195,9 @@ __device__ int round(const P& Pt, Lane<T>& L, V3<T> pa, V3<T> pb, const d3d_mpr_
     case kV2: {  // :198-210; the reference's row swap (:232-240) keeps row 1
                  // as a NumPy view, so both rows end up holding the old row 2
         Pt.set(2, pa, pb, L.d);
-        if (dot(Pt.v(2), L.d) < eps) return kMiss;
+        if (lt(dot(Pt.v(2), L.d), eps)) return kMiss;
         L.d = norm_vector(cross(Pt.v(1) - v0, Pt.v(2) - v0));
-        if (dot(L.d, v0) > T(0)) {
+        if (above0(dot(L.d, v0))) {
             Pt.copy(1, 2);
             L.d = L.d * T(-1);
         }
@@ -208,13 +208,13 @@ __device__ int round(const P& Pt, Lane<T>& L, V3<T> pa, V3<T> pb, const d3d_mpr_
     case kDiscover: {  // :145-158, :213-229
         Pt.set(3, pa, pb, L.d);
         const V3<T> v3 = Pt.v(3);
-        if (dot(v3, L.d) < eps) return kMiss;
+        if (lt(dot(v3, L.d), eps)) return kMiss;
         bool cont = false;
-        if (dot(cross(Pt.v(1), v3), v0) < eps) {
+        if (lt(dot(cross(Pt.v(1), v3), v0), eps)) {
             Pt.copy(2, 3);
             cont = true;
         }
-        if (!cont && dot(cross(v3, Pt.v(2)), v0) < eps) {
+        if (!cont && lt(dot(cross(v3, Pt.v(2)), v0), eps)) {
             Pt.copy(1, 3);
             cont = true;
         }
@@ -225,7 +225,7 @@ __device__ int round(const P& Pt, Lane<T>& L, V3<T> pa, V3<T> pb, const d3d_mpr_
     }
     case kRefine: {  // :243-273, bounded
         const V3<T> v4 = pa - pb;
-        if (!(dot(v4, L.d) > T(-10.0 * kEps)) || reach_tolerance(Pt, v4, L.d, opt.tolerance)) return kMiss;
+        if (!lt(T(-10.0 * kEps), dot(v4, L.d)) || reach_tolerance(Pt, v4, L.d, opt.tolerance)) return kMiss;
         if (L.it >= opt.refine_limit) {
             status = D3D_STATUS_MAX_ITER;
             return kMiss;
@@ -233,7 +233,7 @@ __device__ int round(const P& Pt, Lane<T>& L, V3<T> pa, V3<T> pb, const d3d_mpr_
         expand(Pt, pa, pb, L.d);
         ++L.it;
         L.d = portal_direction(Pt);
-        if (!(dot(Pt.v(1), L.d) > T(-10.0 * kEps))) return kRunning;
+        if (!lt(T(-10.0 * kEps), dot(Pt.v(1), L.d))) return kRunning;
         break;  // the origin is inside
     }
     default: {  // kPenetrate, :320-334
