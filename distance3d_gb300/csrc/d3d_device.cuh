@@ -67,6 +67,7 @@ struct Compare {
     static __device__ __forceinline__ bool below0(T x) { return x < T(0); }
     static __device__ __forceinline__ bool not_below0(T x) { return x >= T(0); }
     static __device__ __forceinline__ bool not_above0(T x) { return x <= T(0); }
+    static __device__ __forceinline__ bool is_zero(T x) { return x == T(0); }
     static __device__ __forceinline__ bool lt_sq(T a, T b) { return a < b; }
     static __device__ __forceinline__ bool le_sq(T a, T b) { return a <= b; }
 };
@@ -100,7 +101,8 @@ struct Compare<double> {
     static __device__ __forceinline__ bool not_above0(double x) {
         return bits(x) - 0x8000000000000000ull <= (unsigned long long)kInf || bits(x) == 0ull;
     }
-    // operands that are +0 or above, or NaN (without a sign): squared lengths
+    static __device__ __forceinline__ bool is_zero(double x) { return (bits(x) << 1) == 0ull; }
+    // operands that are +0 or above, or NaN: squared lengths
     static __device__ __forceinline__ bool lt_sq(double a, double b) {
         return bits(a) < bits(b) && bits(b) <= (unsigned long long)kInf;
     }
@@ -121,6 +123,8 @@ template <typename T>
 __device__ __forceinline__ bool not_below0(T x) { return Compare<T>::not_below0(x); }
 template <typename T>
 __device__ __forceinline__ bool not_above0(T x) { return Compare<T>::not_above0(x); }
+template <typename T>
+__device__ __forceinline__ bool is_zero(T x) { return Compare<T>::is_zero(x); }
 // a < b, a <= b of values that are +0, above, or NaN
 template <typename T>
 __device__ __forceinline__ bool lt_sq(T a, T b) { return Compare<T>::lt_sq(a, b); }

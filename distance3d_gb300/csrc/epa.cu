@@ -48,7 +48,7 @@ __device__ __forceinline__ void st(double* p, d3 v) {
 // utils.py:12-30 norm_vector
 __device__ __forceinline__ d3 norm_vec(d3 v) {
     double n = sqrt(dot(v, v));
-    if (n == 0.0) return v;
+    if (is_zero(n)) return v;
     return mk(v.x / n, v.y / n, v.z / n);
 }
 
@@ -332,20 +332,19 @@ struct WarpPoly {
     __device__ d3 vert(int v) const { return ld(V + 3 * v); }
     __device__ d3 corner(int f, int j) const { return vert((fid[f] >> (8 * j)) & 0xff); }
     __device__ d3 normal(int f) const { return ld(N + 3 * f); }
-    // epa.py:104-106, np.sum(v0 * n) over the face's row
-    __device__ double dist(int f) const {
-        const d3 v = corner(f, 0), n = normal(f);
-        return (v.x * n.x + v.y * n.y) + v.z * n.z;
-    }
 };
 
 // Ordering key of a face distance: unsigned order equals the order of the
 // doubles (-0 as +0); NaN sorts last.
 __device__ __forceinline__ unsigned long long dist_key(double d) {
-    if (d != d) return ~0ull;
-    if (d == 0.0) d = 0.0;
     const unsigned long long u = (unsigned long long)__double_as_longlong(d);
+    if ((u << 1) > 0xffe0000000000000ull) return ~0ull;
+    if ((u << 1) == 0ull) return 0x8000000000000000ull;
     return (u >> 63) ? ~u : (u | 0x8000000000000000ull);
+}
+// The distance of a key (-0 comes back as +0).
+__device__ __forceinline__ double key_dist(unsigned long long k) {
+    return __longlong_as_double((long long)((k >> 63) ? (k == ~0ull ? k : (k & 0x7fffffffffffffffull)) : ~k));
 }
 
 // The warp's smallest (key, index): the smallest key, then the smallest index
@@ -371,12 +370,42 @@ __device__ __forceinline__ unsigned long long max_key(double x) {
 
 // First maximum of V . d over a box's or hull's vertices by the 16 lanes of
 // this half warp (np.argmax): a NaN at vertex 0 wins, later NaNs never do.
+// One FP32 pass bounds the products (hull_argmax_filtered); where one vertex
+// alone can reach the maximum, as nearly always, no FP64 product is taken.
 __device__ __forceinline__ int half_first_max(const d3d_store& st, const Col<double>& c, d3 dd, unsigned half) {
     const int h = lane_of() & 15;
+    if (c.nv == 1) return 0;
+    const Filter32 f = filter32(dd);
+    float lo = -INFINITY, top = -INFINITY, second = -INFINITY;
+    int ti = 0;
+    bool fin = isfinite(f.dabs);
+    for (int k = h; k < c.nv; k += 16) {
+        const float2 se = filter_product(st.verts32, c.off + k, f);
+        fin &= isfinite(se.x) && isfinite(se.y);
+        lo = fmaxf(lo, se.x - se.y);
+        const float up = se.x + se.y;
+        if (up > top) {
+            second = top;
+            top = up;
+            ti = k;
+        } else {
+            second = fmaxf(second, up);
+        }
+    }
+#pragma unroll
+    for (int m = 8; m; m >>= 1) lo = fmaxf(lo, __shfl_xor_sync(half, lo, m));
+    const bool finite = __all_sync(half, fin);
+    const unsigned cand = __ballot_sync(half, top >= lo);
+    const bool many = __any_sync(half, second >= lo);
+    if (finite && !many && __popc(cand) == 1) return __shfl_sync(half, ti, __ffs(cand) - 1);
     unsigned long long bk = 0ull;
     int bj = 0x7fffffff;
     bool nan0 = false;
     for (int k = h; k < c.nv; k += 16) {
+        if (finite) {
+            const float2 se = filter_product(st.verts32, c.off + k, f);
+            if (se.x + se.y < lo) continue;
+        }
         const d3 v = load_vertex(st.verts64, c.off + k);
         const unsigned long long key = max_key(dot102(v.x, v.y, v.z, dd.x, dd.y, dd.z));
         if (k == 0 && key == 0ull) nan0 = true;
@@ -385,6 +414,7 @@ __device__ __forceinline__ int half_first_max(const d3d_store& st, const Col<dou
             bj = k;
         }
     }
+    __syncwarp(half);
     for (int m = 8; m; m >>= 1) {
         const unsigned long long ok = __shfl_xor_sync(half, bk, m);
         const int oi = __shfl_xor_sync(half, bj, m);
@@ -394,7 +424,7 @@ __device__ __forceinline__ int half_first_max(const d3d_store& st, const Col<dou
         }
     }
     const bool any_nan0 = __ballot_sync(half, nan0) != 0u;
-    return (c.nv == 1 || any_nan0 || bj >= c.nv) ? 0 : bj;
+    return (any_nan0 || bj >= c.nv) ? 0 : bj;
 }
 
 // w = s_a(d) - s_b(-d) with the reference's supports: lanes 0-15 evaluate
@@ -414,8 +444,6 @@ __device__ d3 minkowski_exact_warp(const d3d_store& st, int a, int b, d3 d) {
         if (c.nv < 1) {
             s = mk(double(NAN), double(NAN), double(NAN));
         } else {
-            // (The FP32 filter of hull_argmax_filtered does not pay here: with 16 lanes a typical
-            // hull takes a few FP64 rounds, about what its FP32 passes and reductions cost.)
             s = add_margin(c, load_vertex(st.verts64, c.off + half_first_max(st, c, dd, half)), dd);
         }
     } else {
@@ -440,7 +468,7 @@ __device__ int epa_pair_warp(const d3d_store& store, int a, int b, const double*
     __syncwarp();
     {
         const d3 d = ld(P.V + 3 * ((ln >> 2) & 3)) - ld(P.V + 3 * (ln & 3));
-        const unsigned m = __ballot_sync(kWarpAll, ln < 16 && dot(d, d) < lb.edge);
+        const unsigned m = __ballot_sync(kWarpAll, ln < 16 && lt_sq(dot(d, d), lb.edge));
         if (ln < 4) P.pm[ln * P.W] = (m >> (4 * ln)) & 0xfu;
     }
     // epa.py:56-57, 89-97: faces ABC, ACD, ADB, BDC
@@ -481,11 +509,11 @@ __device__ int epa_pair_warp(const d3d_store& store, int a, int b, const double*
         }
         warp_min_key(bk, bi);
         closest = (K[0] == ~0ull || bk == ~0ull) ? 0 : bi;
-        const double md = P.dist(closest);
+        const double md = key_dist(K[closest]);
         const d3 sd = P.normal(closest);
         const d3 w = minkowski_exact_warp(store, a, b, sd);
         const double pd = dot(w, sd);
-        if (pd - md < eps) {  // epa.py:67-70
+        if (lt(pd - md, eps)) {  // epa.py:67-70
             mtv = sd * pd;
             nf_out = nf;
             return D3D_STATUS_OK;
@@ -499,7 +527,7 @@ __device__ int epa_pair_warp(const d3d_store& store, int a, int b, const double*
             bool c = false;
             if (k <= wv) {
                 const d3 d = (k == wv ? w : ld(P.V + 3 * k)) - w;
-                c = dot(d, d) < lb.edge;
+                c = lt_sq(dot(d, d), lb.edge);
             }
             const unsigned m = __ballot_sync(kWarpAll, c);
             if (ln == 0) P.pm[wv * P.W + (kb >> 5)] = m;
@@ -510,7 +538,7 @@ __device__ int epa_pair_warp(const d3d_store& store, int a, int b, const double*
             }
         }
         // epa.py:157-165: visibility of every face (epa.py:122-124)
-        for (int i = ln; i < nf; i += 32) vis[i] = dot(P.normal(i), w - P.corner(i, 0)) > eps ? 1 : 0;
+        for (int i = ln; i < nf; i += 32) vis[i] = lt(eps, dot(P.normal(i), w - P.corner(i, 0))) ? 1 : 0;
         __syncwarp();
         // remove visible faces in the reference's order, collecting edges
         int ne = 0, i = 0;
@@ -581,10 +609,10 @@ __device__ int epa_pair_warp(const d3d_store& store, int a, int b, const double*
                 const d3 e0 = P.vert(ev & 0xffu), e1 = P.vert((ev >> 8) & 0xffu);
                 v0 = e0;
                 nrm = norm_vec(cross(e1 - e0, w - e0));
-                keep = !(dot(nrm, nrm) < lb.keep);
+                keep = !lt_sq(dot(nrm, nrm), lb.keep);
                 // epa.py:139-146: the reference swaps through a NumPy view of
                 // row 0, so the net effect is v0 := v1 (v1 unchanged), n := -n
-                if (keep && dot(v0, nrm) + 1e-6 < 0.0) {
+                if (keep && below0(dot(v0, nrm) + 1e-6)) {
                     v0 = e1;
                     nrm = -nrm;
                     ids = (ids & ~0xffu) | ((ids >> 8) & 0xffu);
@@ -682,22 +710,95 @@ __global__ void k_epa_exact_warp(d3d_store s, const int32_t* __restrict__ i1, co
 // ~8 of 32 lanes active).  Here each round every warp runs one iteration of
 // its pair up to the support, posts the supports of its analytic colliders
 // (a box or hull keeps its 16-lane FP64 argmax in the owning warp), and the
-// posted supports are evaluated one per lane, the supports of collider type t
-// by warp t % W (so that the warps run different types' paths side by side,
-// 61.8 -> 59.1 ms against warp 0 for all); after the visible faces are
-// removed every warp posts its loose edges (up to 32) and all lanes of the
+// posted supports are evaluated on eight lanes each, four per warp
+// (merged_support); after the visible faces are removed every warp posts its loose edges (up to 32) and all lanes of the
 // block compute the new faces' normals, one per lane; each warp then commits
 // its new faces in loose-edge order.  Every value is computed by the same
 // expressions as in epa_pair_warp, so the results are the same bit for bit.
 // A warp whose pair ends (or that has none) sits out the rest of the round.
+//
+// Polytopes of up to 64 faces (and pairs without close vertices) keep the
+// visibility flags and the loose edges in registers while the visible faces are
+// removed: 600 -> ~200 cycles per face.  6,007 pairs at the default limits 1110
+// us (13.3M FP64 warp instructions, supports 43%) -> 846 us (8.7M);
+// 20,000 pairs at 256 faces 4.26 -> 3.49 ms.  Left out: an FP32 bound before
+// the visibility and closeness tests (7.4M FP64 instructions, but 935 us: a
+// round waits for instructions issued, not for the pipe), 20 and 24 warps per SM
+// (1004 and 981 against 971 us before the register loose list).
 
 constexpr int kFaceTaskPerWarp = 32;  // loose edges a warp posts per round; more are computed in place
+
+__device__ __forceinline__ double group_at(double x, int j) { return __shfl_sync(kWarpAll, x, j, 8); }
+
+// Component j = lane & 7 (j < 3; lanes 3-7 repeat component 0) of the support
+// along d of an analytic collider (not a box, hull or MeshGraph), eight lanes
+// per collider, four colliders of any types per warp; all 32 lanes call it.
+// support() of one lane is a chain of 45-65 FP64 instructions, and a warp with
+// several types runs one chain after the other.  Here the types share one
+// chain -- the pose products, one square root, one division, the way back to
+// the world -- with the three components side by side: ~36 instructions for
+// any four colliders.  Every value is computed by base_support's and
+// add_margin's expressions in their order.
+__device__ __forceinline__ double merged_support(const d3d_store& st, int idx, d3 d) {
+    const int4 meta = __ldg(reinterpret_cast<const int4*>(st.meta) + idx);
+    const int ty = meta.x;
+    const int j = lane_of() & 7, i = j < 3 ? j : 0;
+    const bool sphere = ty == D3D_SPHERE, capsule = ty == D3D_CAPSULE, cylinder = ty == D3D_CYLINDER;
+    const bool disk = ty == D3D_DISK, cone = ty == D3D_CONE, ellipse = ty == D3D_ELLIPSE, ellipsoid = ty == D3D_ELLIPSOID;
+    const bool vec = sphere || ellipsoid || ellipse;  // types that divide a vector by its norm
+    const double* rec = st.rec64 + (size_t)idx * 16;
+    const double t = __ldg(rec + 9 + i), p0 = __ldg(rec + 12), p1 = __ldg(rec + 13);
+    const double pi = sphere ? p0 : __ldg(rec + 12 + i);
+    const double c0 = __ldg(rec + i), c1 = __ldg(rec + 3 + i), c2 = __ldg(rec + 6 + i);            // R's column i
+    const double r0 = __ldg(rec + 3 * i), r1 = __ldg(rec + 3 * i + 1), r2 = __ldg(rec + 3 * i + 2);  // and row i
+    const double di = i == 0 ? d.x : (i == 1 ? d.y : d.z);
+    // local direction: R^T d in gemv order, a disk's in ddot order (its third component unused), a
+    // sphere's d itself
+    double l = fma(c2, d.z, fma(disk ? c1 : c0, disk ? d.y : d.x, (disk ? c0 : c1) * (disk ? d.x : d.y)));
+    if (sphere) l = di;
+    if (disk && i == 2) l = 0.0;
+    // the vector whose norm is taken, and the norm in the type's order
+    const double w = ellipsoid || ellipse ? l * pi : l;
+    const double sq = w * w;
+    const double xx = group_at(sq, 0), wy = group_at(w, 1), wz = group_at(w, 2);
+    const double f1 = fma(wy, wy, xx), f2 = fma(wz, wz, f1);
+    const double u1 = xx + group_at(sq, 1), u2 = u1 + group_at(sq, 2);
+    const double n = sqrt(capsule ? u2 : (cylinder ? u1 : (sphere || ellipsoid ? f2 : f1)));
+    const bool zero = is_zero(n);
+    double v;
+    if (!zero) {
+        const double q = (vec ? w : p0) / n;
+        v = q * (vec ? pi : (cone && i == 2 ? 0.0 : l));  // (w / n) * p, or l * (p0 / n)
+    } else if (ellipsoid || ellipse) {
+        v = w * pi;
+    } else {
+        v = (capsule || cylinder) && i == 0 ? p0 : (sphere && i == 2 ? p0 : 0.0);
+    }
+    const double h = 0.5 * p1;
+    if (i == 2 && capsule) v = v + (above0(l) ? h : -h);
+    if (i == 2 && cylinder) v = below0(l) ? -h : h;
+    __syncwarp();
+    double vx = group_at(v, 0), vy = group_at(v, 1), vz = group_at(v, 2);
+    const double lx = group_at(l, 0), ly = group_at(l, 1), lz = group_at(l, 2);
+    if (cone && !le(lz * p1, dot012(lx, ly, lz, vx, vy, vz))) {  // the tip
+        vx = vy = 0.0;
+        vz = p1;
+    }
+    double x = ellipse ? fma(vy, r1, vx * r0) : dot102(r0, r1, r2, vx, vy, vz);
+    if (sphere) x = v;
+    x = t + x;
+    if (disk && zero) x = t;
+    if (meta.w) {
+        const double m = sqrt(dot(d, d));
+        x = x + __ldg(rec + 15) * (is_zero(m) ? di : di / m);
+    }
+    return x;
+}
 
 struct BlockTasks {
     double* sres;            // support results, 3 doubles per task (task 2 w + side)
     double* sdir;            // support directions of the posted tasks
     int* scol;               // collider of each posted task, -1 if none
-    int* stype;              // its collider type
     double* fn;              // new faces: normal (3 doubles) per task
     unsigned long long* fk;  // their distance keys (kept faces)
     unsigned* fid;           // ids | 1 << 31 if kept
@@ -709,7 +810,7 @@ struct BlockTasks {
 __host__ __device__ inline int block_task_bytes(int W) {
     const int st = 2 * W;
     const int ft = W * kFaceTaskPerWarp;
-    return ((st * 48 + st * 8 + ft * (24 + 8 + 4 + 4) + W * 4 + 16) + 15) & ~15;
+    return ((st * 48 + st * 4 + ft * (24 + 8 + 4 + 4) + W * 4 + 16) + 15) & ~15;
 }
 
 template <int W>
@@ -721,8 +822,7 @@ __device__ __forceinline__ BlockTasks block_tasks_at(unsigned char* base) {
     T.fn = T.sdir + 3 * ST;
     T.fk = reinterpret_cast<unsigned long long*>(T.fn + 3 * FT);
     T.scol = reinterpret_cast<int*>(T.fk + FT);
-    T.stype = T.scol + ST;
-    T.fid = reinterpret_cast<unsigned*>(T.stype + ST);
+    T.fid = reinterpret_cast<unsigned*>(T.scol + ST);
     T.ftask = T.fid + FT;
     T.wv = reinterpret_cast<int*>(T.ftask + FT);
     T.nface = T.wv + W;
@@ -739,10 +839,10 @@ __device__ __forceinline__ void new_face(const WarpPoly& P, int k, int wv, Lengt
     const d3 e0 = P.vert(ev & 0xffu), e1 = P.vert((ev >> 8) & 0xffu), w = P.vert(wv);
     v0 = e0;
     nrm = norm_vec(cross(e1 - e0, w - e0));
-    keep = !(dot(nrm, nrm) < lb.keep);
+    keep = !lt_sq(dot(nrm, nrm), lb.keep);
     // epa.py:139-146: the reference swaps through a NumPy view of row 0, so
     // the net effect is v0 := v1 (v1 unchanged), n := -n
-    if (keep && dot(v0, nrm) + 1e-6 < 0.0) {
+    if (keep && below0(dot(v0, nrm) + 1e-6)) {
         v0 = e1;
         nrm = -nrm;
         ids = (ids & ~0xffu) | ((ids >> 8) & 0xffu);
@@ -772,6 +872,7 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_epa_exact_block(d3d_store s,
     int64_t pid = 0;
     int a = 0, b = 0, nf = 0, closest = 0, nv = 0, it = 0, stt = 0;
     bool have = false, exhausted = false;
+    bool dup = false;  // two vertices are close (or one not even to itself): edges match through pm
     d3 mtv = mk(0.0, 0.0, 0.0);
     // The block's shared work (posted supports, new faces) goes to warps by a rotation that
     // changes every round and differs between the blocks of an SM, so that it does not always
@@ -809,8 +910,9 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_epa_exact_block(d3d_store s,
             __syncwarp();
             {
                 const d3 d = ld(P.V + 3 * ((ln >> 2) & 3)) - ld(P.V + 3 * (ln & 3));
-                const unsigned m = __ballot_sync(kWarpAll, ln < 16 && dot(d, d) < lb.edge);
+                const unsigned m = __ballot_sync(kWarpAll, ln < 16 && lt_sq(dot(d, d), lb.edge));
                 if (ln < 4) P.pm[ln * P.W] = (m >> (4 * ln)) & 0xfu;
+                dup = m != 0x8421u;
             }
             if (ln < 4) {
                 const int init[4][3] = {{0, 1, 2}, {0, 2, 3}, {0, 3, 1}, {1, 3, 2}};
@@ -854,7 +956,7 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_epa_exact_block(d3d_store s,
             }
             warp_min_key(bk, bi);
             closest = (K[0] == ~0ull || bk == ~0ull) ? 0 : bi;
-            md = P.dist(closest);
+            md = key_dist(K[closest]);
             sd = P.normal(closest);
             // supports: a box or hull by its half warp here (first maximum of V . d, a NaN at vertex
             // 0 wins, later NaNs never do); the other types are posted for warp 0
@@ -878,22 +980,30 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_epa_exact_block(d3d_store s,
             } else if ((ln & 15) == 0) {
                 st(T.sdir + 3 * (2 * wp + side), dd);
                 T.scol[2 * wp + side] = up ? b : a;
-                T.stype[2 * wp + side] = c.type;
             }
         } else if (ln < 2) {
             T.scol[2 * wp + ln] = -1;
         }
         __syncthreads();
-        // the posted supports, one per lane, each collider type on its own warp where W allows
-        // (the analytic types numbered 0-7, rotated), so that the warps run different types'
-        // FP64 paths side by side
-        if (ln < 2 * W) {
-            const int ci = T.scol[ln];
-            const int ty = T.stype[ln];
-            if (ci >= 0 && (ty - (ty > D3D_BOX) - (ty > D3D_HULL) + rot) % W == wp) {
-                Col<double> c;
-                load_col(s, ci, c);
-                st(T.sres + 3 * ln, support(c, s, ld(T.sdir + 3 * ln)));
+        // the posted supports, four to a warp, the warps in turn
+        {
+            const int part = wp - rot + (wp < rot ? W : 0);  // tasks 4 part .. 4 part + 3
+            if (4 * part < 2 * W) {
+                const int task = 4 * part + (ln >> 3);
+                const int ci = T.scol[task];
+                const bool on = ci >= 0;
+                int type = -1, nv, off;
+                if (on) load_meta(s, ci, type, nv, off);
+                const d3 dd = ld(T.sdir + 3 * task);
+                if (__any_sync(kWarpAll, on && type != D3D_MESH)) {
+                    const double x = merged_support(s, on ? ci : 0, dd);
+                    if (on && type != D3D_MESH && (ln & 7) < 3) T.sres[3 * task + (ln & 7)] = x;
+                }
+                if (type == D3D_MESH && (ln & 7) == 0) {
+                    Col<double> c;
+                    load_col(s, ci, c);
+                    st(T.sres + 3 * task, support(c, s, dd));
+                }
             }
         }
         __syncthreads();
@@ -902,7 +1012,7 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_epa_exact_block(d3d_store s,
         if (run) {
             w = ld(T.sres + 3 * (2 * wp)) - ld(T.sres + 3 * (2 * wp + 1));
             const double pd = dot(w, sd);
-            if (pd - md < eps) {  // epa.py:67-70
+            if (lt(pd - md, eps)) {  // epa.py:67-70
                 mtv = sd * pd;
                 stt = D3D_STATUS_OK;
                 run = false;
@@ -919,9 +1029,10 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_epa_exact_block(d3d_store s,
                 bool c = false;
                 if (k <= wv) {
                     const d3 d = (k == wv ? w : ld(P.V + 3 * k)) - w;
-                    c = dot(d, d) < lb.edge;
+                    c = lt_sq(dot(d, d), lb.edge);
                 }
                 const unsigned m = __ballot_sync(kWarpAll, c);
+                dup |= m != ((wv >> 5) == (kb >> 5) ? 1u << (wv & 31) : 0u);
                 if (ln == 0) P.pm[wv * P.W + (kb >> 5)] = m;
                 if (k < wv) {
                     unsigned& word = P.pm[k * P.W + (wv >> 5)];
@@ -930,58 +1041,130 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_epa_exact_block(d3d_store s,
                 }
             }
             // epa.py:157-165: visibility of every face (epa.py:122-124)
-            for (int i = ln; i < nf; i += 32) vis[i] = dot(P.normal(i), w - P.corner(i, 0)) > eps ? 1 : 0;
-            __syncwarp();
-            // remove visible faces in the reference's order, collecting edges
-            int i = 0;
-            while (true) {
-                int p = -1;
-                for (int base = i; base < nf; base += 32) {
-                    const int j = base + ln;
-                    const unsigned m = __ballot_sync(kWarpAll, j < nf && vis[j]);
-                    if (m) {
-                        p = base + __ffs(m) - 1;
-                        break;
-                    }
+            if (nf <= 64 && !dup) {
+                // up to 64 faces: their flags in a register; no two vertices close: edges match by
+                // their ids, and the loose list sits in registers too, edge k on lane k
+                unsigned long long seen = 0;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int f = 32 * h + ln;
+                    bool v = false;
+                    if (32 * h < nf && f < nf) v = lt(eps, dot(P.normal(f), w - P.corner(f, 0)));
+                    if (32 * h < nf) seen |= (unsigned long long)__ballot_sync(kWarpAll, v) << (32 * h);
                 }
-                if (p < 0) break;
-                const unsigned fv = P.fid[p];
-                for (int j = 0; j < 3; ++j) {
-                    const int x0 = (fv >> (8 * j)) & 0xff, x1 = (fv >> (8 * ((j + 1) % 3))) & 0xff;
-                    int found = -1;
-                    for (int kb = 0; kb < ne; kb += 32) {
-                        const int k = kb + ln;
-                        bool match = false;
-                        if (k < ne) {
-                            const unsigned e = P.eid[k];
-                            match = P.close(e >> 8, x0) && P.close(e & 0xff, x1);
+                const int limit = o.max_loose_edges;
+                unsigned mine = 0;  // this lane's loose edge: a | b << 8
+                bool spilled = false;
+                while (seen) {
+                    // the lowest visible face: the reference scans on from the slot it filled last
+                    const int p = __ffsll((long long)seen) - 1;
+                    const unsigned fv = P.fid[p];
+                    if (ne > 29 && !spilled) {  // the list may outgrow the lanes: on in shared memory
+                        if (ln < ne) P.eid[ln] = (unsigned short)mine;
+                        spilled = true;
+                        __syncwarp();
+                    }
+                    for (int j = 0; j < 3; ++j) {
+                        const unsigned x0 = (fv >> (8 * j)) & 0xff, x1 = (fv >> (8 * ((j + 1) % 3))) & 0xff;
+                        const unsigned want = x1 | (x0 << 8);  // the loose edge (x1, x0)
+                        int found = -1;
+                        if (!spilled) {
+                            const unsigned m = __ballot_sync(kWarpAll, ln < ne && mine == want);
+                            if (m) found = __ffs(m) - 1;
+                        } else {
+                            for (int kb = 0; kb < ne && found < 0; kb += 32) {
+                                const int k = kb + ln;
+                                const unsigned m = __ballot_sync(kWarpAll, k < ne && P.eid[k] == want);
+                                if (m) found = kb + __ffs(m) - 1;
+                            }
                         }
-                        const unsigned m = __ballot_sync(kWarpAll, match);
+                        if (found >= 0) {
+                            if (!spilled) {
+                                const unsigned last = __shfl_sync(kWarpAll, mine, ne - 1);
+                                if (ln == found) mine = last;
+                            } else if (ln == 0) {
+                                P.eid[found] = P.eid[ne - 1];
+                            }
+                            --ne;
+                        } else {
+                            if (ne >= limit) break;  // epa.py:193-198
+                            if (!spilled) {
+                                if (ln == ne) mine = x0 | (x1 << 8);
+                            } else if (ln == 0) {
+                                P.eid[ne] = (unsigned short)(x0 | (x1 << 8));
+                            }
+                            ++ne;
+                        }
+                        if (spilled) __syncwarp();
+                    }
+                    // epa.py:118-120: the last face moves into slot p, which is tested again
+                    if (ln < 3) P.N[3 * p + ln] = P.N[3 * (nf - 1) + ln];
+                    if (ln == 0) {
+                        K[p] = K[nf - 1];
+                        P.fid[p] = P.fid[nf - 1];
+                    }
+                    --nf;
+                    const unsigned long long moved = (seen >> nf) & 1ull;
+                    seen &= ~((1ull << nf) | (1ull << p));
+                    if (p < nf) seen |= moved << p;
+                    __syncwarp();
+                }
+                if (!spilled && ln < ne) P.eid[ln] = (unsigned short)mine;
+                __syncwarp();
+            } else {
+                for (int i = ln; i < nf; i += 32) vis[i] = lt(eps, dot(P.normal(i), w - P.corner(i, 0))) ? 1 : 0;
+                __syncwarp();
+                // remove visible faces in the reference's order, collecting edges
+                int i = 0;
+                while (true) {
+                    int p = -1;
+                    for (int base = i; base < nf; base += 32) {
+                        const int j = base + ln;
+                        const unsigned m = __ballot_sync(kWarpAll, j < nf && vis[j]);
                         if (m) {
-                            found = kb + __ffs(m) - 1;
+                            p = base + __ffs(m) - 1;
                             break;
                         }
                     }
-                    if (found >= 0) {
-                        if (ln == 0) P.eid[found] = P.eid[ne - 1];
-                        --ne;
-                    } else {
-                        if (ne >= o.max_loose_edges) break;  // epa.py:193-198
-                        if (ln == 0) P.eid[ne] = (unsigned short)(x0 | (x1 << 8));
-                        ++ne;
+                    if (p < 0) break;
+                    const unsigned fv = P.fid[p];
+                    for (int j = 0; j < 3; ++j) {
+                        const int x0 = (fv >> (8 * j)) & 0xff, x1 = (fv >> (8 * ((j + 1) % 3))) & 0xff;
+                        int found = -1;
+                        for (int kb = 0; kb < ne; kb += 32) {
+                            const int k = kb + ln;
+                            bool match = false;
+                            if (k < ne) {
+                                const unsigned e = P.eid[k];
+                                match = P.close(e >> 8, x0) && P.close(e & 0xff, x1);
+                            }
+                            const unsigned m = __ballot_sync(kWarpAll, match);
+                            if (m) {
+                                found = kb + __ffs(m) - 1;
+                                break;
+                            }
+                        }
+                        if (found >= 0) {
+                            if (ln == 0) P.eid[found] = P.eid[ne - 1];
+                            --ne;
+                        } else {
+                            if (ne >= o.max_loose_edges) break;  // epa.py:193-198
+                            if (ln == 0) P.eid[ne] = (unsigned short)(x0 | (x1 << 8));
+                            ++ne;
+                        }
+                        __syncwarp();
                     }
+                    // epa.py:118-120: the last face moves into slot p, which is tested again
+                    if (ln < 3) P.N[3 * p + ln] = P.N[3 * (nf - 1) + ln];
+                    if (ln == 0) {
+                        vis[p] = vis[nf - 1];
+                        K[p] = K[nf - 1];
+                        P.fid[p] = P.fid[nf - 1];
+                    }
+                    --nf;
+                    i = p;
                     __syncwarp();
                 }
-                // epa.py:118-120: the last face moves into slot p, which is tested again
-                if (ln < 3) P.N[3 * p + ln] = P.N[3 * (nf - 1) + ln];
-                if (ln == 0) {
-                    vis[p] = vis[nf - 1];
-                    K[p] = K[nf - 1];
-                    P.fid[p] = P.fid[nf - 1];
-                }
-                --nf;
-                i = p;
-                __syncwarp();
             }
         }
         // the new faces of up to 32 loose edges per warp go to the block
