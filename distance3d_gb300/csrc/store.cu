@@ -3,6 +3,7 @@
 // value here must match the reference's FP64 rounding sequence.
 #include "capi_util.h"
 #include "d3d_device.cuh"
+#include "scratch.h"
 
 namespace {
 
@@ -459,15 +460,18 @@ extern "C" int d3d_store_pack(const d3d_store* store, const int32_t* types, cons
                 "d3d_store_pack: n_hull_vertices %lld outside [0, %lld]", (long long)n_hull_vertices,
                 (long long)store->n_vertices);
     cudaStream_t st = d3d::as_stream(stream);
-    int* bad = nullptr;
-    if (cudaMallocAsync(&bad, sizeof(int), st) != cudaSuccess || cudaMemsetAsync(bad, 0, sizeof(int), st) != cudaSuccess)
-        return d3d::check_launch("d3d_store_pack: flag");
+    // from the library's pool: the default pool gives its memory back at every synchronisation
+    void* block = nullptr;
+    rc = d3d::scratch_alloc(&block, sizeof(int), st);
+    if (rc) return rc;
+    int* const bad = static_cast<int*>(block);
+    cudaMemsetAsync(bad, 0, sizeof(int), st);
     if (n_hull_vertices > 0) k_hull_to_f32<<<d3d::grid_for(n_hull_vertices, 256), 256, 0, st>>>(*store, n_hull_vertices);
     if (n > 0)
         k_pack<<<d3d::grid_for(n, 128), 128, 0, st>>>(*store, types, poses, params, hull_offset, hull_count, n, bad);
     int hbad = 0;
     cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, st);
-    cudaFreeAsync(bad, st);
+    d3d::scratch_free(block, st);
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
         d3d::set_error("d3d_store_pack: %s", cudaGetErrorString(e));

@@ -100,6 +100,17 @@ def _pair_store(collider1, collider2):
     return ColliderStore(ColliderSet.from_colliders([collider1, collider2]))
 
 
+def _one_pair(store):
+    """Index tensors of the pair (0, 1), and distance outputs in one buffer,
+    so that one copy brings them to the host: (i1, i2, out, buffer)."""
+    pair = torch.arange(2, dtype=torch.int32, device=store.device)
+    buf = torch.empty(256, dtype=torch.uint8, device=store.device)
+    d = buf[:152].view(torch.float64)
+    out = dict(dist=d[:1], cp1=d[1:4], cp2=d[4:7], simplex=d[7:19], iterations=buf[152:156].view(torch.int32),
+               n_simplex=buf[156:157], status=buf[157:158])
+    return pair[:1], pair[1:], out, buf
+
+
 def _mesh_cache_holder(c):
     """The object that holds a MeshGraph collider's vertex cache (``first_idx``):
     this package's MeshGraph, or the support object of distance3d's own
@@ -127,21 +138,23 @@ def gjk_distance_jolt(collider1, collider2, tolerance=1e-10, max_distance_square
     if any(x is not None for x in holders):
         cache = torch.tensor([[int(x.first_idx) if x is not None else -1 for x in holders]], dtype=torch.int32,
                              device=store.device)
-    r = gjk_distance_batch(store, [0], [1], tolerance=tolerance, max_distance_squared=max_distance_squared,
-                           sanity_check=sanity_check, mesh_cache=cache)
-    h = {k: v.cpu().numpy() for k, v in r.items()}
+    i1, i2, out, buf = _one_pair(store)
+    gjk_distance_batch(store, i1, i2, tolerance=tolerance, max_distance_squared=max_distance_squared,
+                       sanity_check=sanity_check, mesh_cache=cache, out=out)
+    h = buf.cpu().numpy()
+    d = h[:152].view(np.float64)
     if cache is not None:
         for x, v in zip(holders, cache.cpu().numpy()[0]):
             if x is not None:
                 x.first_idx = int(v)
-    status = int(h["status"][0])
+    status = int(h[157])
     if status == _lib.STATUS_CLIPPED:
         return MAX_FLOAT, None, None, None
     if status == _lib.STATUS_SANITY:
         raise AssertionError("Sanity check failed")
     if status == _lib.STATUS_MAX_ITER:
         raise RuntimeError("GJK did not converge within the iteration bound")
-    return float(h["dist"][0]), h["cp1"][0], h["cp2"][0], h["simplex"][0]
+    return float(d[0]), d[1:4].copy(), d[4:7].copy(), d[7:19].reshape(4, 3).copy()
 
 
 def gjk_intersection_jolt(collider1, collider2, tolerance=1e-10):

@@ -48,6 +48,23 @@ def as_index(x, device, n=None):
     return torch.as_tensor(np.ascontiguousarray(a, dtype=np.int32), device=device)
 
 
+# Arrays of a collider set up to this size in all reach the device in one copy: a pageable copy takes
+# ~16 us however small, while copying larger arrays together first costs the host more than it saves.
+STAGE_BYTES = 1 << 16
+
+
+def _staged(arrays, device):
+    """One device copy of several host arrays: (tensor of bytes, offsets)."""
+    offsets, total = [], 0
+    for a in arrays:
+        offsets.append(total)
+        total += (a.nbytes + 255) & ~255
+    host = np.zeros(total, np.uint8)
+    for a, o in zip(arrays, offsets):
+        host[o:o + a.nbytes] = a.reshape(-1).view(np.uint8)
+    return torch.from_numpy(host).to(device), offsets
+
+
 class PinnedColliderSet:
     """A ColliderSet staged in page-locked host memory, so that building a
     store from it is a set of asynchronous host-to-device copies."""
@@ -114,22 +131,28 @@ class ColliderStore:
             self.rec64 = torch.empty((max(n, 1), 16), dtype=torch.float64, device=dev)
             self.rec32 = torch.empty((max(n, 1), 16), dtype=torch.float32, device=dev)
             self.meta = torch.empty((max(n, 1), 4), dtype=torch.int32, device=dev)
-            self.verts64 = torch.zeros((max(n_vertices, 1), 4), dtype=torch.float64, device=dev)
             self.verts32 = torch.empty((max(n_vertices, 1), 4), dtype=torch.float32, device=dev)
-            if nv_hull:
-                self.verts64[:nv_hull].copy_(torch.from_numpy(cs.vertices))
-            self.links = torch.from_numpy(cs.links).to(dev) if len(cs.links) else None
-            types = torch.from_numpy(cs.types).to(dev)
-            poses = torch.from_numpy(cs.poses).to(dev)
-            params = torch.from_numpy(cs.params).to(dev)
-            offs = torch.from_numpy(offsets).to(dev)
-            cnts = torch.from_numpy(counts).to(dev)
+            small = (cs.types, cs.poses, cs.params, offsets, counts)
+            rows = max(n_vertices, 1)
+            if sum(x.nbytes for x in small) + 32 * rows + cs.links.nbytes <= STAGE_BYTES:
+                verts = np.zeros((rows, 4))
+                verts[:nv_hull] = cs.vertices
+                stage, at = _staged(small + (verts, cs.links), dev)
+                ptrs = [ctypes.c_void_p(stage.data_ptr() + o) for o in at[:5]]
+                self.verts64 = stage[at[5]:at[5] + verts.nbytes].view(torch.float64).view(rows, 4)
+                self.links = stage[at[6]:at[6] + cs.links.nbytes].view(torch.int32) if len(cs.links) else None
+            else:
+                self.verts64 = torch.zeros((rows, 4), dtype=torch.float64, device=dev)
+                if nv_hull:
+                    self.verts64[:nv_hull].copy_(torch.from_numpy(cs.vertices))
+                self.links = torch.from_numpy(cs.links).to(dev) if len(cs.links) else None
+                stage = [torch.from_numpy(x).to(dev) for x in small]
+                ptrs = [_ptr(t) for t in stage]
             self._view = _lib.D3DStore(n, n_vertices, self.rec64.data_ptr(), self.rec32.data_ptr(),
                                        self.meta.data_ptr(), self.verts64.data_ptr(), self.verts32.data_ptr(),
                                        self.links.data_ptr() if self.links is not None else None,
                                        len(cs.links))
-            _lib.check(lib.d3d_store_pack(ctypes.byref(self._view), _ptr(types), _ptr(poses), _ptr(params),
-                                          _ptr(offs), _ptr(cnts), nv_hull, _stream(dev)))
+            _lib.check(lib.d3d_store_pack(ctypes.byref(self._view), *ptrs, nv_hull, _stream(dev)))
 
     def _init_pinned(self, p, device):
         self.device = torch.device(device)
