@@ -20,11 +20,11 @@
 //    origin.  Every other separated or touching pair is flagged, its FP64 rows
 //    in its record, and a stable compaction (CUB) lists the flagged pairs in
 //    the type-sorted order.
-// B  continues the reference's loop in FP64 for the listed pairs, one round
-//    per lane and iteration (pb_round): the first round solves the handed
-//    rows, later rounds add a support pair along -v, until the duality gap
-//    closes as in R.  A pair whose loop ends leaves its simplex in the outputs
-//    and the rest of its state in its record.
+// B  continues the reference's loop (_gjk_jolt.py:224-288) in FP64 for the
+//    listed pairs, a pool of pairs per block: the first round solves the
+//    handed rows, later rounds add a support pair along -v, until the duality
+//    gap closes as in R.  A pair whose loop ends leaves its simplex in the
+//    outputs and the rest of its state in its record.
 // E  (the end pass) computes the closest points and the checks of B's
 //    finished pairs (pb_end), every lane on a finished pair.
 // C  is the plain FP64 kernel over the fallback list (the reference's
@@ -34,10 +34,9 @@
 // a warp are active, so the FP64 work sits where lanes are busy: R runs the
 // same support code on every lane of a warp and a short per-lane solve, and
 // only the pairs R cannot finish (those whose gap or feature check fails)
-// pay for B's divergent per-lane loop.  B keeps the simplex P/Q rows in
-// shared memory and has one support call site.  A pair goes to the fallback
-// list only if its result fails the consistency check (closest points vs |v|)
-// or the sanity check in E, or hits the iteration bound in B.
+// pay for B's loop.  A pair goes to the fallback list only if its result fails
+// the consistency check (closest points vs |v|) or the sanity check in E, or
+// hits the iteration bound in B.
 //
 // On the six-type workloads A takes ~11 FP32 iterations and R evaluates ~3
 // rows plus the gap row, against ~17-19 FP64 iterations for the plain form.
@@ -50,6 +49,7 @@
 #include "gjk_impl.h"
 #include "gjk_mixed.cuh"
 #include "gjk_out.cuh"
+#include "gjk_pool.cuh"
 #include "persist.cuh"
 #include "scratch.h"
 
@@ -221,7 +221,7 @@ __device__ __forceinline__ void r_finish(const double* my, int nr, bool sep, boo
         for (int j = 1; j < 3; ++j)
             if (j < nr) ymax = maxf2(ymax, dot(w[j], w[j]));
         const double tol_sq = opt.tolerance * opt.tolerance;
-        // touching in FP64 (pb_round's test) is B's to decide
+        // touching in FP64 (B's test) is B's to decide
         const bool apart = vl > tol_sq && vl > DBL_EPSILON * ymax;
         const bool closed = gap <= kMixedRelGap * upper || gap * gap <= kMixedAbsGap2 * maxf2(1.0, dot(wg, wg));
         if (inside && apart && closed) {
@@ -464,85 +464,296 @@ __global__ void __launch_bounds__(BLOCK) k_gjk_mixed_r(d3d_store s, const int32_
     }
 }
 
-// B over R's run list, in the type-sorted order.
-template <int BLOCK, bool MESH>
-__global__ void __launch_bounds__(BLOCK) k_gjk_mixed_b(d3d_store s, const int32_t* __restrict__ i1,
-                                                        const int32_t* __restrict__ i2, d3d_gjk_options opt,
-                                                        const Handoff* __restrict__ hand, DistanceOut o, Lists lists) {
-    __shared__ double rows[24 * BLOCK];
-    const int64_t n = (int64_t)lists.ctr[kNumRun];
-    // a short list is spread over the grid's warps: its lanes would run their pairs' different
-    // paths one after the other
-    if ((int)(threadIdx.x & 31) >= spread_lanes(n, BLOCK)) return;
+// B over R's run list, in the type-sorted order: a pool of S pairs per block
+// in shared memory, in rounds as the plain FP64 GJK runs them (gjk_pool.cuh,
+// whose pool it uses).  Each round lists the pairs' supports by collider type
+// (a hull is searched by the whole warp) and, after the new Minkowski points,
+// the simplices by size, and the lanes of a warp take one kind.  A pair's
+// first round (the replay) solves the handed-over rows without a support.
+// The arithmetic is RefineSupport's and closest_to_origin's as they compile
+// for one lane per pair.  With one lane per pair this kernel had 5.4 lanes per
+// FP64 instruction: 87,819 scene pairs 385 -> 361 us, 300,032 robot pairs
+// 356 -> 299 us, 20,011 pairs of ten types 222 -> 187 us, 3,000 pairs 120 ->
+// 107 us, 1M pairs 727 -> 720 us.
+constexpr int kReplay = 3;  // state beside pool::kFree, kLive
+
+template <int S>
+__device__ __forceinline__ void b_finish(const pool::Mem<S, 4>& m, int s, unsigned perm, int n, d3 dir, double vl,
+                                         int state, const Handoff* hand, const DistanceOut& o, const Lists& lists) {
+    // the closest points and checks (pb_end) run in the end pass
+    const int pid = m.pid[s];
+    EndRecord& e = lists.records[pid];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (k < n) {
+            const int r = pool::place_of(perm, k);
+            const d3 pk = m.row(m.P, r, s), qk = m.row(m.Q, r, s);
+            e.pq[k][0] = pk.x;
+            e.pq[k][1] = pk.y;
+            e.pq[k][2] = pk.z;
+            e.pq[k][3] = qk.x;
+            e.pq[k][4] = qk.y;
+            e.pq[k][5] = qk.z;
+        }
+    }
+    e.dir[0] = dir.x;
+    e.dir[1] = dir.y;
+    e.dir[2] = dir.z;
+    e.vl = vl;
+    e.it = m.it[s] + handoff_iters(hand[pid].v);
+    e.state = state;
+    e.status = D3D_STATUS_OK;
+    e.n = n;
+    double* sp = o.simplex + 12 * (int64_t)pid;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const d3 y = m.row(m.Y, pool::place_of(perm, j), s);
+        sp[3 * j] = y.x;
+        sp[3 * j + 1] = y.y;
+        sp[3 * j + 2] = y.z;
+    }
+    o.n_simplex[pid] = (int8_t)n;
+    append_warp(lists.ends, lists.ctr + kNumEnd, true, pid);
+}
+
+template <int S, bool MESH>
+__global__ void __launch_bounds__(S, 3) k_gjk_mixed_b(d3d_store st, const int32_t* __restrict__ i1,
+                                                            const int32_t* __restrict__ i2, d3d_gjk_options opt,
+                                                            const Handoff* __restrict__ hand, DistanceOut o,
+                                                            Lists lists) {
+    constexpr unsigned kAll = 0xffffffffu;
+    constexpr int kBins = 2 * kSupportTypes;
+    extern __shared__ __align__(16) unsigned char b_smem[];
+    pool::Mem<S, 4>& m = *reinterpret_cast<pool::Mem<S, 4>*>(b_smem);
+    const int t = threadIdx.x, ln = t & 31;
+    const long long n = (long long)lists.ctr[kNumRun];
     const JoltEps<double> E = reference_eps<double>();
     const double tol_sq = opt.tolerance * opt.tolerance;
-    PhaseB<SmemRows<double, BLOCK>> B;
-    B.g.S.R.base = rows + threadIdx.x;
-    int32_t pid = 0;
-    int a = 0, b = 0;
-    int it_a = 0;
-    bool need = true;
-    unsigned live = __activemask();  // the warp's lanes still in the loop
+    const long long share = (n + gridDim.x - 1) / gridDim.x;
+    const long long split = share < S ? 0 : n;
+    bool exhausted = t >= share;
     WarpChunk chunk;
-    // per-lane claims for the last slots: the pairs are short, and slots left in a busy warp's chunk
-    // would hold up the end of the launch
-    const long long split = n - 2LL * gridDim.x * blockDim.x;
-    while (true) {
-        __syncwarp(live);
-        const long long slot = fetch_slot_chunked(lists.ctr + kCurB, need, chunk, live, kChunk, split);
-        const bool quit = need && slot >= n;
-        live = __ballot_sync(live, !quit);
-        if (quit) break;
-        if (need) {
-            pid = lists.run[slot];
-            a = i1[pid];
-            b = i2[pid];
-            it_a = handoff_iters(hand[pid].v);
-            pb_begin(B, lists.records[pid]);
-            need = false;
-        }
-        __syncwarp(live);  // the round starts converged (pb_round keeps it so through the solve)
-        if (B.mode == PB_FALLBACK || pb_round<MESH>(B, s, a, b, tol_sq, opt, E)) {
-            if (B.mode != PB_FALLBACK) {
-                // The closest points and checks of the pair (pb_end) run in
-                // the end pass, where a warp's lanes all hold finished pairs;
-                // here only a few lanes finish per round.
-                const GjkLoop<double, SmemRows<double, BLOCK>>& g = B.g;
-                EndRecord& e = lists.records[pid];
+    m.meta[t] = 0;
+    if (t < kBins) m.cnt[0][t] = m.cnt[1][t] = 0;
+    if (t < 4) m.scnt[0][t] = m.scnt[1][t] = m.next[t >> 1][t & 1] = 0;
+    int type[2] = {0, 0};
+    __syncthreads();
+    for (int par = 0;; par ^= 1) {
+        // ---- free slots take new pairs
+        int state = pool::meta_state(m.meta[t]);
+        const bool want = state == pool::kFree && !exhausted;
+        const long long slot = fetch_slot_chunked(lists.ctr + kCurB, want, chunk, kAll, kChunk, split);
+        if (want) {
+            if (slot >= n) {
+                exhausted = true;
+            } else {
+                const int pid = lists.run[slot];
+                const EndRecord& rec = lists.records[pid];
+                const int rows = rec.n;
+                if (rows < 1 || rows > 4) {
+                    lists.fallback[atomicAdd(lists.ctr + kNumFallback, 1ull)] = pid;
+                } else {
+                    m.pid[t] = pid;
+                    m.it[t] = 0;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    if (k < g.S.n) {
-                        const d3 pk = g.S.R.p(k), qk = g.S.R.q(k);
-                        e.pq[k][0] = pk.x;
-                        e.pq[k][1] = pk.y;
-                        e.pq[k][2] = pk.z;
-                        e.pq[k][3] = qk.x;
-                        e.pq[k][4] = qk.y;
-                        e.pq[k][5] = qk.z;
+                    for (int k = 0; k < 2; ++k) {
+                        const int c = (k ? i2 : i1)[pid];
+                        const int4 q = __ldg(reinterpret_cast<const int4*>(st.meta) + c);
+                        type[k] = support_bin(q.x, q.w);
+                        m.col[k * S + t] = c;
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        d3 y = mk(0.0, 0.0, 0.0);
+                        if (j < rows) {
+                            const d3 p = mk(rec.pq[j][0], rec.pq[j][1], rec.pq[j][2]);
+                            const d3 q = mk(rec.pq[j][3], rec.pq[j][4], rec.pq[j][5]);
+                            m.put(m.P, j, t, p);
+                            m.put(m.Q, j, t, q);
+                            y = p - q;
+                        }
+                        m.put(m.Y, j, t, y);
+                    }
+                    m.meta[t] = pool::pack_meta(0xe4u, rows, 0, kReplay);
+                    state = kReplay;
+                }
+            }
+        }
+        // ---- list the supports
+        int pos[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int bin = state == pool::kLive ? type[k] : -1;
+            const unsigned same = __match_any_sync(kAll, bin);
+            const int leader = __ffs(same) - 1;
+            int base = 0;
+            if (ln == leader && bin >= 0) base = atomicAdd(&m.cnt[par][bin], __popc(same));
+            pos[k] = __shfl_sync(kAll, base, leader) + __popc(same & ((1u << ln) - 1u));
+        }
+        if (!__syncthreads_or(state != pool::kFree || !exhausted)) break;
+        const Chunks ch = chunks_of(m.cnt[par], kBins, (ln >> 1) == D3D_HULL ? pool::kHullChunk : 32);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int p = ch.start(type[k]) + pos[k];
+            if (state == pool::kLive) m.list[p] = (unsigned short)(2 * t + k);
+        }
+        __syncthreads();
+        int cb, first, count;
+        while (ch.take(&m.next[par][0], cb, first, count)) {
+            const bool on = ln < count;
+            const int e = m.list[first + (on ? ln : 0)];
+            const int s = e >> 1, side = e & 1;
+            const int c = m.col[side * S + s];
+            d3 d = m.direction(s);
+            if (side) d = -d;
+            const f3 df = RefineSupportT<MESH>::rounded(d);
+            int vi = -1;
+            if ((cb >> 1) == D3D_HULL) {
+                int ty, nv, off;
+                load_meta(st, c, ty, nv, off);
+                for (int h = 0; h < count; ++h) {
+                    const int w = warp_hull_argmax(
+                        st.verts32, __shfl_sync(kAll, off, h), max(__shfl_sync(kAll, nv, h), 1),
+                        mk(__shfl_sync(kAll, df.x, h), __shfl_sync(kAll, df.y, h), __shfl_sync(kAll, df.z, h)));
+                    if (ln == h) vi = w;
+                }
+            }
+            if (on) {
+                Col<double> cl;
+                load_col(st, c, cl);
+                m.put_support(s, side, RefineSupportT<MESH>::eval_at(cl, st, d, df, vi));
+            }
+            __syncwarp();
+        }
+        __syncthreads();
+        // ---- advance
+        int cls = -1;
+        if (state == kReplay) {
+            cls = 4 - pool::meta_n(m.meta[t]);
+        } else if (state == pool::kLive) {
+            const unsigned mt = m.meta[t];
+            const unsigned perm = mt & 0xffu;
+            const int f = pool::meta_fresh(mt), rows = pool::meta_n(mt);
+            const int it = m.it[t];
+            bool fallback = it >= opt.max_iterations;
+            if (!fallback) {
+                m.it[t] = it + 1;
+                const d3 w = m.row(m.P, f, t) - m.row(m.Q, f, t);
+                const d3 dir = m.direction(t);
+                const double vl = m.vl[t];
+                const double dd = dot(dir, w);
+                // duality gap: |v| - (|v|^2 - v.w) / |v| <= distance <= |v|
+                const double gap = vl + dd;
+                if (dd < 0.0 && dd * dd > vl * opt.max_distance_squared) {
+                    fallback = true;  // clipped: the FP64 kernel reports it
+                } else if (rows > 0 &&
+                           (gap <= kMixedRelGap * vl || gap * gap <= kMixedAbsGap2 * maxf2(1.0, dot(w, w)) * vl)) {
+                    b_finish(m, t, perm, rows, -dir, vl, GJK_NO_INTERSECTION, hand, o, lists);
+                    m.meta[t] = 0;
+                } else {
+                    m.put(m.Y, f, t, w);
+                    m.meta[t] = pool::pack_meta((perm & ~(3u << (2 * rows))) | ((unsigned)f << (2 * rows)), rows + 1,
+                                                0, pool::kLive);
+                    cls = 3 - rows;
+                }
+            }
+            if (fallback) {
+                lists.fallback[atomicAdd(lists.ctr + kNumFallback, 1ull)] = m.pid[t];
+                m.meta[t] = 0;
+            }
+        }
+        __syncwarp();
+        {
+            unsigned mine = 0;
+            int base = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const unsigned b = __ballot_sync(kAll, cls == k);
+                if (cls == k) mine = b;
+                if (ln == k) base = b ? atomicAdd(&m.scnt[par][k], __popc(b)) : 0;
+            }
+            const int p = __shfl_sync(kAll, base, cls >= 0 ? cls : 0) + __popc(mine & ((1u << ln) - 1u));
+            if (cls >= 0) m.solve[cls * S + p] = (unsigned short)t;
+        }
+        if (t < kBins) m.cnt[par ^ 1][t] = 0;
+        if (t < 4) m.scnt[par ^ 1][t] = 0;
+        if (t < 2) m.next[par ^ 1][t] = 0;
+        __syncthreads();
+        // ---- solve, 16 simplices of one size to a chunk
+        const Chunks ph = chunks_of(m.scnt[par], 4, 16);
+        while (ph.take(&m.next[par][1], cb, first, count)) {
+            const int k0 = first - ph.start(cb);
+            if (ln < count) {
+                const int s = m.solve[cb * S + k0 + ln];
+                const unsigned mt = m.meta[s];
+                const bool replay = pool::meta_state(mt) == kReplay;
+                unsigned perm = mt & 0xffu;
+                Simplex<double, RegRows<double>> X;
+                X.n = pool::meta_n(mt);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) X.Y[k] = m.y(mt, k, s);
+                double prev = replay ? DBL_MAX : m.prev[s];
+                d3 nv;
+                double nl;
+                int set;
+                d3 dir;
+                double vl;
+                bool fallback = false;
+                if (closest_to_origin<double, RegRows<double>, true>(X, prev, E, nv, nl, set)) {
+                    dir = nv;
+                    vl = nl;
+                } else if (replay) {
+                    fallback = true;
+                } else {
+                    --X.n;
+                    set = (1 << X.n) - 1;
+                    dir = m.direction(s);
+                    vl = m.vl[s];
+                }
+                int ended = -1;
+                if (fallback) {
+                    lists.fallback[atomicAdd(lists.ctr + kNumFallback, 1ull)] = m.pid[s];
+                    m.meta[s] = 0;
+                } else if (set == 15) {
+                    vl = 0.0;
+                    ended = GJK_INTERSECTION;
+                } else {
+                    unsigned np = perm;
+                    int k = 0;
+                    double y = 0.0;
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        if (r < X.n && ((set >> r) & 1)) {
+                            np = (np & ~(3u << (2 * k))) | (((perm >> (2 * r)) & 3u) << (2 * k));
+                            const double l = dot(X.Y[r], X.Y[r]);
+                            if (k == 0 || l > y) y = l;
+                            ++k;
+                        }
+                    perm = np;
+                    X.n = k;
+                    if (vl <= tol_sq || vl <= E.isect * y) {
+                        vl = 0.0;
+                        ended = GJK_INTERSECTION;
+                    } else {
+                        dir = -dir;
+                        if (prev - vl <= E.conv * prev) ended = GJK_NO_INTERSECTION;
                     }
                 }
-                e.dir[0] = g.dir.x;
-                e.dir[1] = g.dir.y;
-                e.dir[2] = g.dir.z;
-                e.vl = g.vl;
-                e.it = g.it + it_a;
-                e.state = g.state;
-                e.status = g.status;
-                e.n = g.S.n;
-                double* sp = o.simplex + 12 * (int64_t)pid;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    sp[3 * j] = g.S.Y[j].x;
-                    sp[3 * j + 1] = g.S.Y[j].y;
-                    sp[3 * j + 2] = g.S.Y[j].z;
+                if (ended >= 0) {
+                    b_finish(m, s, perm, X.n, dir, vl, ended, hand, o, lists);
+                    m.meta[s] = 0;
+                } else if (!fallback) {
+                    m.prev[s] = vl;
+                    m.vl[s] = vl;
+                    m.dir[s] = dir.x;
+                    m.dir[S + s] = dir.y;
+                    m.dir[2 * S + s] = dir.z;
+                    m.meta[s] = pool::pack_meta(perm, X.n, pool::free_place(perm, X.n), pool::kLive);
                 }
-                o.n_simplex[pid] = (int8_t)g.S.n;
-                append_warp(lists.ends, lists.ctr + kNumEnd, true, pid);
-            } else {
-                lists.fallback[atomicAdd(lists.ctr + kNumFallback, 1ull)] = pid;
             }
-            need = true;
+            __syncwarp();
         }
+        __syncthreads();
     }
 }
 
@@ -611,6 +822,9 @@ size_t gjk_mixed_scratch_bytes(int64_t capacity) {
            select_temp_bytes(capacity);
 }
 
+// B's pairs (and threads) per block
+constexpr int kLoopPool = 128;
+
 // R's block: 30 doubles of shared memory per lane
 constexpr int kRefineBlock = 128;
 
@@ -648,9 +862,18 @@ int launch_mixed(const d3d_store& store, const int32_t* i1, const int32_t* i2, c
         set_error("d3d_gjk_distance (mixed, run list): %s", cudaGetErrorString(e));
         return D3D_ERR_CUDA;
     }
-    const void* kb = (const void*)k_gjk_mixed_b<BLOCK, MESH>;
-    k_gjk_mixed_b<BLOCK, MESH><<<persistent_blocks(kb, BLOCK, 32 * n, per_sm), BLOCK, 0, stream>>>(store, i1, i2, opt,
-                                                                                             hand, o, lists);
+    const void* kb = (const void*)k_gjk_mixed_b<kLoopPool, MESH>;
+    const int smem = (int)sizeof(pool::Mem<kLoopPool, 4>);
+    e = cudaFuncSetAttribute(kb, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kb, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 (int)cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) {
+        set_error("d3d_gjk_distance (mixed, FP64 loop): %s", cudaGetErrorString(e));
+        return D3D_ERR_CUDA;
+    }
+    k_gjk_mixed_b<kLoopPool, MESH><<<persistent_blocks(kb, kLoopPool, n * kLoopPool, 0, smem), kLoopPool, smem, stream>>>(
+        store, i1, i2, opt, hand, o, lists);
     rc = check_launch("d3d_gjk_distance (mixed, FP64 loop)");
     if (rc) return rc;
     k_gjk_mixed_end<<<persistent_blocks((const void*)k_gjk_mixed_end, 128, 32 * n), 128, 0, stream>>>(opt, o, lists);

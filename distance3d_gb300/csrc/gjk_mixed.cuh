@@ -413,7 +413,7 @@ __device__ __forceinline__ Handoff pa_handoff(const PhaseALoop<Rows>& L, int out
 }
 
 // ---------------------------------------------------------------- phase B
-enum PhaseBMode { PB_RUN = 0, PB_DONE = 1, PB_FALLBACK = 2, PB_REPLAY = 3 };
+enum PhaseBEnd { PB_DONE = 1, PB_FALLBACK = 2 };
 
 // The FP64 rows of one pair that the refinement pass hands to B: the support
 // points p and q of each row of A's final simplex, evaluated in FP64 along
@@ -428,119 +428,6 @@ struct alignas(16) EndRecord {
     int status;
     int n;
 };
-
-// FP64 continuation of the reference's loop for one pair, a per-lane state
-// machine.  REPLAY: the simplex holds the FP64 rows handed over by the
-// refinement pass, and the first round solves it as the loop's first
-// iteration would (nothing to beat yet).  If it encloses or touches the
-// origin the pair is done; otherwise RUN continues the reference's loop from
-// there, stopped by the duality gap.
-template <typename Rows>
-struct PhaseB {
-    GjkLoop<double, Rows> g;
-    int mode;
-};
-
-template <typename Rows>
-__device__ __forceinline__ void pb_begin(PhaseB<Rows>& B, const EndRecord& rec) {
-    simplex_clear(B.g.S);
-    B.g.it = 0;
-    B.g.state = GJK_RUNNING;
-    B.g.status = D3D_STATUS_OK;
-    const int n = rec.n;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        if (j < n) {
-            const d3 p = mk(rec.pq[j][0], rec.pq[j][1], rec.pq[j][2]);
-            const d3 q = mk(rec.pq[j][3], rec.pq[j][4], rec.pq[j][5]);
-            simplex_push(B.g.S, p - q, p, q);
-        }
-    }
-    B.mode = n > 0 && n <= 4 ? PB_REPLAY : PB_FALLBACK;
-}
-
-// One round for one lane: nothing to evaluate in the REPLAY round (the rows
-// are in the simplex), one FP64 support pair along the loop's direction in a
-// RUN round, then the simplex update (_gjk_jolt.py:224-288).  Every round ends
-// in the simplex solve, so a warp's lanes reach it together whatever mode
-// each is in.  Returns true once the loop has ended: g.state is
-// GJK_INTERSECTION or GJK_NO_INTERSECTION (pb_end finishes the pair), or
-// B.mode is PB_FALLBACK (clipped, iteration bound, failed replay).
-template <bool MESH = true, typename Rows>
-__device__ __forceinline__ bool pb_round(PhaseB<Rows>& B, const d3d_store& s, int a, int b, double tol_sq,
-                                         const d3d_gjk_options& opt, const JoltEps<double>& E) {
-    GjkLoop<double, Rows>& g = B.g;
-    const bool replay = B.mode == PB_REPLAY;
-    // The lanes that call together solve together: the support and its
-    // checks only set `ended`, and all lanes reconverge before the solve (see
-    // gjk_step).
-    const unsigned together = __activemask();
-    int ended = 0;  // 1: to the fallback (iteration bound, clipped); 2: the duality gap closed
-    if (!replay) {
-        if (g.it >= opt.max_iterations) {
-            ended = 1;
-        } else {
-            ++g.it;
-            d3 p, q;
-            pair_supports<double, RefineSupportT<MESH>>(s, a, b, g.dir, p, q);
-            const d3 w = p - q;
-            const double dd = dot(g.dir, w);
-            // duality gap: |v| - (|v|^2 - v.w) / |v| <= distance <= |v|
-            const double gap = g.vl + dd;
-            if (dd < 0.0 && dd * dd > g.vl * opt.max_distance_squared) {
-                ended = 1;  // clipped: the FP64 kernel reports it
-            } else if (g.S.n > 0 && (gap <= kMixedRelGap * g.vl ||
-                                     gap * gap <= kMixedAbsGap2 * maxf2(1.0, dot(w, w)) * g.vl)) {
-                g.dir = -g.dir;
-                g.state = GJK_NO_INTERSECTION;
-                ended = 2;
-            } else {
-                simplex_push(g.S, w, p, q);
-            }
-        }
-    }
-    __syncwarp(together);
-    if (ended) {
-        if (ended == 1) B.mode = PB_FALLBACK;
-        return true;
-    }
-    d3 nv;
-    double nl;
-    int set;
-    const double prev = replay ? DBL_MAX : g.prev;
-    if (closest_to_origin<double, Rows, true>(g.S, prev, E, nv, nl, set)) {
-        g.dir = nv;
-        g.vl = nl;
-    } else if (replay) {
-        B.mode = PB_FALLBACK;
-        return true;
-    } else {
-        --g.S.n;
-        set = (1 << g.S.n) - 1;
-    }
-    if (replay) {
-        B.mode = PB_RUN;
-        g.prev = DBL_MAX;
-    }
-    if (set == 15) {
-        g.vl = 0.0;
-        g.state = GJK_INTERSECTION;
-        return true;
-    }
-    simplex_compact<double, true>(g.S, set);
-    if (g.vl <= tol_sq || g.vl <= E.isect * max_y_len_sq(g.S)) {
-        g.vl = 0.0;
-        g.state = GJK_INTERSECTION;
-        return true;
-    }
-    g.dir = -g.dir;
-    if (g.prev - g.vl <= E.conv * g.prev) {
-        g.state = GJK_NO_INTERSECTION;
-        return true;
-    }
-    g.prev = g.vl;
-    return false;
-}
 
 // ---------------------------------------------------------------- refinement pass
 // Closest point to the origin of the affine hull of the rows w[0..n), n <= 3,
