@@ -42,8 +42,10 @@ size_t gjk_bytes(int64_t capacity, const d3d_gjk_options& g) {
 }
 
 // Every pair k < n gets "no EPA" (status -1, NaN mtv, no faces); those GJK
-// left at distance 0 with a full simplex are appended to the EPA list.
-__global__ void k_epa_select(int64_t cap, const int64_t* __restrict__ n_dev, const double* __restrict__ dist,
+// left at distance 0 with a full simplex are appended to the EPA list, in
+// about the type-sorted order if GJK had one (order, else null).
+__global__ void k_epa_select(int64_t cap, const int64_t* __restrict__ n_dev, const int32_t* __restrict__ order,
+                             const double* __restrict__ dist,
                              const int8_t* __restrict__ n_simplex, int32_t* __restrict__ list,
                              unsigned long long* __restrict__ count, double* __restrict__ mtv,
                              int8_t* __restrict__ status, int32_t* __restrict__ n_faces) {
@@ -51,15 +53,17 @@ __global__ void k_epa_select(int64_t cap, const int64_t* __restrict__ n_dev, con
     for (int64_t k0 = (int64_t)blockIdx.x * blockDim.x; k0 < cap; k0 += (int64_t)gridDim.x * blockDim.x) {
         const int64_t k = k0 + threadIdx.x;
         bool take = false;
+        int64_t q = k;
         if (k < n) {
             mtv[3 * k] = NAN;
             mtv[3 * k + 1] = NAN;
             mtv[3 * k + 2] = NAN;
             status[k] = -1;
             n_faces[k] = 0;
-            take = dist[k] == 0.0 && n_simplex[k] == 4;
+            if (order) q = order[k];
+            take = dist[q] == 0.0 && n_simplex[q] == 4;
         }
-        append_warp(list, count, take, (int32_t)k);
+        append_warp(list, count, take, (int32_t)q);
     }
 }
 
@@ -118,12 +122,13 @@ extern "C" int d3d_collide(const d3d_store* store, const int32_t* i1, const int3
         return D3D_ERR_CUDA;
     }
     DistanceOut o{dist, cp1, cp2, simplex, n_simplex, status, iterations};
+    const int32_t* order = nullptr;
     rc = gjk->precision == D3D_PRECISION_MIXED
-             ? d3d::gjk_mixed_run(*store, i1, i2, capacity, n_dev, *gjk, o, gjk_scratch, st)
+             ? d3d::gjk_mixed_run(*store, i1, i2, capacity, n_dev, *gjk, o, gjk_scratch, st, &order)
              : d3d::gjk_f64_run(*store, i1, i2, capacity, n_dev, *gjk, o, gjk_scratch, st);
     if (rc) return rc;
     const int sel_blocks = d3d::persistent_blocks((const void*)k_epa_select, kBlock, capacity);
-    k_epa_select<<<sel_blocks, kBlock, 0, st>>>(capacity, n_dev, dist, n_simplex, list, ctr + kNumEpa, mtv,
+    k_epa_select<<<sel_blocks, kBlock, 0, st>>>(capacity, n_dev, order, dist, n_simplex, list, ctr + kNumEpa, mtv,
                                                 epa_status, n_faces);
     rc = d3d::check_launch("d3d_collide (EPA pair selection)");
     if (rc) return rc;

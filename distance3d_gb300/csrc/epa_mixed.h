@@ -22,16 +22,16 @@ int epa_mixed_launch(const d3d_store& store, const int32_t* i1, const int32_t* i
                      int8_t* status, int32_t* n_faces, double* faces, void* scratch, int64_t max_slots,
                      int32_t* fallback, unsigned long long* n_fallback, cudaStream_t stream);
 
-// The warp-per-pair form (epa_warp.cu): one warp per pair, its polytope in
+// The form with the lanes of a warp on a pair (epa_warp.cu), its polytope in
 // shared memory, FP32 (fp64 = false) or FP64 with the reference's supports
 // (fp64 = true, for the FP32 form's fallback pairs); supported when
-// max_iterations <= 250, max_loose_edges <= 255 and four polytopes fit in a
-// block's shared memory.  Runs pairs list[k] (or k) for k < n, or
+// max_iterations <= 250, max_loose_edges <= 255 and two polytopes of a whole
+// warp fit in a block's shared memory.  Runs pairs list[k] (or k) for k < n, or
 // k < *n_dev if n_dev is given (n then only sizes the launch); fallback pairs
-// as above.  With `refine` (FP32 form only), each converged pair's FP32 face
-// normal goes to mtv and the pair to refine[*n_refine ...] (the caller zeroes
-// the count), and a second kernel then computes the pairs' FP64 depths along
-// those normals, one pair per thread.
+// as above.  The FP32 form writes each converged pair's FP32 face normal to
+// mtv and the pair to refine[*n_refine ...] (the caller zeroes the count, the
+// FP64 form takes neither), and a second kernel then computes the pairs' FP64
+// depths along those normals, one pair per thread.
 bool epa_warp_supported(const d3d_epa_options& o, bool fp64 = false);
 int epa_warp_launch(const d3d_store& store, const int32_t* i1, const int32_t* i2, const int32_t* list, int64_t n,
                     const unsigned long long* n_dev, unsigned long long* cursor, const double* simplex,

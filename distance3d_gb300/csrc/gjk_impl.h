@@ -17,10 +17,12 @@ int launch_gjk_f64(const d3d_store& store, const int32_t* i1, const int32_t* i2,
 
 // The mixed form on caller scratch (gjk_mixed_scratch_bytes(n)); with n_dev,
 // the pair count is *n_dev <= n, read on the device, and the launches depend
-// on n only (a CUDA graph can hold them).
+// on n only (a CUDA graph can hold them).  `sorted`, if not null, receives the
+// type-sorted order of the pairs in `scratch` (null: the batch was not sorted).
 size_t gjk_mixed_scratch_bytes(int64_t capacity);
 int gjk_mixed_run(const d3d_store& store, const int32_t* i1, const int32_t* i2, int64_t n, const int64_t* n_dev,
-                  const d3d_gjk_options& opt, const DistanceOut& o, void* scratch, cudaStream_t stream);
+                  const d3d_gjk_options& opt, const DistanceOut& o, void* scratch, cudaStream_t stream,
+                  const int32_t** sorted = nullptr);
 
 // the same on the FP64 kernel (gjk.cu)
 size_t gjk_f64_scratch_bytes(int64_t capacity);

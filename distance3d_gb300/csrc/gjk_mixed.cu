@@ -893,7 +893,8 @@ int launch_mixed(const d3d_store& store, const int32_t* i1, const int32_t* i2, c
 }
 
 int gjk_mixed_run(const d3d_store& store, const int32_t* i1, const int32_t* i2, int64_t n, const int64_t* n_dev,
-                  const d3d_gjk_options& opt, const DistanceOut& o, void* scratch, cudaStream_t stream) {
+                  const d3d_gjk_options& opt, const DistanceOut& o, void* scratch, cudaStream_t stream,
+                  const int32_t** sorted) {
     const d3d_tuning t = tuning();
     const bool sched = n >= t.sort_min;
     const size_t c = (size_t)n;
@@ -904,6 +905,7 @@ int gjk_mixed_run(const d3d_store& store, const int32_t* i1, const int32_t* i2, 
     lists.ctr = reinterpret_cast<unsigned long long*>(p);
     p += 256;
     int32_t* order = sched ? reinterpret_cast<int32_t*>(p) : nullptr;
+    if (sorted) *sorted = order;
     p += order_bytes;
     void* temp = p;
     p += temp_bytes;
