@@ -41,31 +41,32 @@ METRIC = "GJK+EPA pairs/s (mixed precision form; plain FP64 form alongside)"
 UNIT = "pairs/s"
 EPA_KW = dict(max_iter=64, max_loose_edges=128, max_faces=256, epsilon=1e-8)
 # DRAM bytes per pair of the mixed kernels from one ncu capture of the
-# 131,072-pair workload (k_gjk_mixed_a + _r + _b + _end per pair; k_epa_warp
-# + k_epa_refine per EPA pair, 38,814 of them); traffic grows in proportion
-# to the pairs
-NCU_DRAM_BYTES_PER_PAIR = {"gjk_mixed": (78589696 + 3613952 + 112622080 + 10178304 + 16011520 + 256 + 7312384
-                                         + 185600) / 131072,
-                           "epa_mixed": (33024000 + 32512 + 34504192 + 13568) / 38814}
+# 131,072-pair workload (k_gjk_mixed_a + _r + _b + _end per pair;
+# k_epa_segments + k_epa_refine per EPA pair, 38,814 of them); traffic grows
+# in proportion to the pairs
+NCU_DRAM_BYTES_PER_PAIR = {"gjk_mixed": (78693376 + 3753728 + 124820736 + 8987904 + 17338880 + 512 + 7130880)
+                           / 131072,
+                           "epa_mixed": (33004288 + 44800 + 38616832 + 37376) / 38814}
 # Pipe and issue activity (fractions of peak, ncu --set full at 131,072
 # pairs) of the mixed kernels, reported beside the model-FLOP fraction: the
 # model counts only the geometry's arithmetic, while the kernels are bound by
 # instruction issue (EPA search) or latency (phase A), and ncu's FMA-pipe
 # share counts every FP32 instruction, compares and selects included
 NCU_PIPE_ACTIVITY = {
-    "gjk_mixed": {"k_gjk_mixed_a": {"fma_pipe": 0.193, "fp64_pipe": 0.0, "issue": 0.451},
-                  "k_gjk_mixed_r": {"fma_pipe": 0.019, "fp64_pipe": 0.686, "issue": 0.102},
-                  "k_gjk_mixed_b": {"fma_pipe": 0.008, "fp64_pipe": 0.503, "issue": 0.089},
-                  "k_gjk_mixed_end": {"fma_pipe": 0.003, "fp64_pipe": 0.488, "issue": 0.050}},
-    "epa_mixed": {"k_epa_warp<float>": {"fma_pipe": 0.230, "fp64_pipe": 0.072, "issue": 0.749},
-                  "k_epa_refine": {"fma_pipe": 0.029, "fp64_pipe": 0.290, "issue": 0.089}}}
+    "gjk_mixed": {"k_gjk_mixed_a": {"fma_pipe": 0.192, "fp64_pipe": 0.0, "issue": 0.449},
+                  "k_gjk_mixed_r": {"fma_pipe": 0.029, "fp64_pipe": 0.565, "issue": 0.146},
+                  "k_gjk_mixed_b": {"fma_pipe": 0.011, "fp64_pipe": 0.455, "issue": 0.076},
+                  "k_gjk_mixed_end": {"fma_pipe": 0.005, "fp64_pipe": 0.747, "issue": 0.078}},
+    "epa_mixed": {"k_epa_segments": {"fma_pipe": 0.171, "fp64_pipe": 0.147, "issue": 0.602},
+                  "k_epa_refine": {"fma_pipe": 0.030, "fp64_pipe": 0.510, "issue": 0.166}}}
 # this library's kernels per timed mixed step (one graph replay), used only
 # when the graph cannot be read back (d3d_graph_kernel_nodes): k_pair_keys,
 # k_gjk_mixed_a, k_gjk_mixed_r, k_gjk_mixed_b, k_gjk_mixed_end,
-# k_gjk_distance_f64 (fallback list), k_epa_select, k_epa_warp<float>,
-# k_epa_refine, k_epa_warp<double> (fallback list), k_epa_exact_warp (second
-# fallback list); the CUB sort and compaction kernels are the toolkit's
-MIXED_STEP_LAUNCHES = 11
+# k_gjk_pool (fallback list), k_epa_select, k_epa_segments (twice: the form for
+# few pairs returns at once), k_epa_refine, k_epa_warp<double> (fallback list),
+# k_epa_exact_block (second fallback list); the CUB sort and compaction kernels
+# are the toolkit's
+MIXED_STEP_LAUNCHES = 12
 
 # Algorithmic bytes per pair (counted once): two collider records, the hull
 # vertices of hull colliders, and the outputs.  FP64 record 120 B (pose 96 +
@@ -930,10 +931,10 @@ def run_ours(args):
     times = {"gjk_mixed": gjk_mixed, "epa_mixed": epa_mixed, "gjk_fp64": gjk_fp64, "epa_fp64": epa_fp64}
     peak_src = "FMA chains measured in this run (libd3d_peak)"
     compute_roofline = {}
-    for key, kernel, peak in (("gjk_fp64", "k_gjk_distance_f64_grouped", peak64),
+    for key, kernel, peak in (("gjk_fp64", "k_gjk_pool", peak64),
                               ("epa_fp64", "k_epa_exact_block", peak64),
                               ("gjk_mixed", "k_gjk_mixed_a/_r/_b/_end", peak32),
-                              ("epa_mixed", "k_epa_warp<float> + k_epa_refine", peak32)):
+                              ("epa_mixed", "k_epa_segments + k_epa_refine", peak32)):
         compute_roofline[key] = {"kernel": kernel, "bound": "fp64 pipe" if peak is peak64 else "fp32 pipe",
                                  "model_flops_per_launch": flops[key], "ms": 1e3 * times[key],
                                  "achieved_tflops": flops[key] / times[key] / 1e12, "peak_tflops": peak / 1e12,
@@ -954,7 +955,7 @@ def run_ours(args):
         dom, key, bytes_dom = "d3d_gjk_distance mixed (k_gjk_mixed_a, _r, _b, _end)", "gjk_mixed", gjk_bytes
         traffic = NCU_DRAM_BYTES_PER_PAIR["gjk_mixed"] * n
     else:
-        dom, key, bytes_dom = "d3d_epa mixed (k_epa_warp<float>, k_epa_refine)", "epa_mixed", epa_bytes
+        dom, key, bytes_dom = "d3d_epa mixed (k_epa_segments, k_epa_refine)", "epa_mixed", epa_bytes
         traffic = NCU_DRAM_BYTES_PER_PAIR["epa_mixed"] * n_epa
     t_dom = times[key]
     hbm = {"achieved": bytes_dom / t_dom / 1e9, "peak": hbm_peak, "unit": "GB/s",

@@ -1356,9 +1356,9 @@ int launch_segments(const d3d_store& store, const int32_t* i1, const int32_t* i2
     const int smem = byte_poly_bytes(o) * WARPS * Seg<W>::kPairs;
     int rc = prepare_smem(fn, smem);
     if (rc) return rc;
-    k_epa_segments<W, WARPS, MESH><<<persistent_blocks(fn, 32 * WARPS, n * 32, 0, smem), 32 * WARPS, smem, stream>>>(
-        store, i1, i2, list, n, n_dev, cursor, simplex, o, mtv, status, n_faces, faces, fallback, n_fallback, refine,
-        n_refine, lo, hi);
+    k_epa_segments<W, WARPS, MESH><<<persistent_blocks(fn, 32 * WARPS, launch_items(n * 32, n * W / 4), 0, smem), 32 * WARPS, smem,
+                                     stream>>>(store, i1, i2, list, n, n_dev, cursor, simplex, o, mtv, status, n_faces,
+                                               faces, fallback, n_fallback, refine, n_refine, lo, hi);
     return check_launch("d3d_epa (mixed)");
 }
 
@@ -1377,9 +1377,9 @@ int launch_search(const d3d_store& store, const int32_t* i1, const int32_t* i2, 
                   const d3d_epa_options& o, double* mtv, int8_t* status, int32_t* n_faces, double* faces,
                   int32_t* fallback, unsigned long long* n_fallback, int32_t* refine, unsigned long long* n_refine,
                   cudaStream_t stream) {
-    const int64_t few = 2 * seg_warps(32) * (int64_t)sm_count() + 1;
+    const int64_t few = shared_gpu() ? 0 : 2 * seg_warps(32) * (int64_t)sm_count() + 1;
     // with the count on the device the forms of both sides are launched and one returns at once
-    if (n_dev || n < few) {
+    if (few && (n_dev || n < few)) {
         const int rc = launch_segments<32, WARPS, MESH>(store, i1, i2, list, n < few ? n : few, n_dev, cursor, simplex,
                                                         o, mtv, status, n_faces, faces, fallback, n_fallback, refine,
                                                         n_refine, 0, few, stream);
@@ -1416,7 +1416,7 @@ int launch_warp(const d3d_store& store, const int32_t* i1, const int32_t* i2, co
     }
     if (rc || sizeof(T) == 8) return rc;
     const void* kr = (const void*)k_epa_refine<MESH>;
-    k_epa_refine<MESH><<<persistent_blocks(kr, kRefine, 8 * n), kRefine, 0, stream>>>(store, i1, i2, refine, n_refine, mtv);
+    k_epa_refine<MESH><<<persistent_blocks(kr, kRefine, launch_items(8 * n, n)), kRefine, 0, stream>>>(store, i1, i2, refine, n_refine, mtv);
     return check_launch("d3d_epa (mixed, refinement)");
 }
 

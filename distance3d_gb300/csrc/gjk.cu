@@ -67,7 +67,7 @@ int launch_pool(const d3d_store& store, const int32_t* i1, const int32_t* i2, co
         return D3D_ERR_CUDA;
     }
     // a block per pair for the smallest batches: their pairs run side by side
-    const int blocks = persistent_blocks(fn, kPool, n * kPool, blocks_per_sm(tuning(), kPool), smem);
+    const int blocks = persistent_blocks(fn, kPool, launch_items(n * kPool, n), blocks_per_sm(tuning(), kPool), smem);
     pool::k_gjk_pool<kPool, PQ><<<blocks, kPool, smem, stream>>>(store, i1, i2, order, n, n_dev, cursor, opt, o, hits);
     return check_launch(PQ == 4 ? "d3d_gjk_distance" : "d3d_gjk_intersection");
 }

@@ -834,8 +834,8 @@ int launch_mixed(const d3d_store& store, const int32_t* i1, const int32_t* i2, c
                  const Lists& lists, void* select_temp, size_t select_bytes, int per_sm, cudaStream_t stream) {
     const float tol_sq = (float)(opt.tolerance * opt.tolerance);
     const void* ka = (const void*)k_gjk_mixed_a<BLOCK, MESH>;
-    const int full = persistent_blocks(ka, BLOCK, 32 * n, per_sm);  // every block the GPU holds, down to a pair per warp
-    if (n >= (int64_t)full * BLOCK)
+    const int full = persistent_blocks(ka, BLOCK, launch_items(32 * n, n), per_sm);  // alone: down to a pair per warp
+    if (shared_gpu() || n >= (int64_t)full * BLOCK)
         k_gjk_mixed_a<BLOCK, MESH><<<full, BLOCK, 0, stream>>>(store, i1, i2, order, n, n_dev, tol_sq,
                                                                (float)opt.max_distance_squared, opt.max_iterations,
                                                                hand, o, lists);
@@ -850,7 +850,7 @@ int launch_mixed(const d3d_store& store, const int32_t* i1, const int32_t* i2, c
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     int64_t per = (n + 2 * sms - 1) / (2 * sms);
-    per = per < 16 ? 16 : (per > kRefineBlock ? kRefineBlock : per);
+    per = per < 16 ? 16 : (per > kRefineBlock || shared_gpu() ? kRefineBlock : per);
     k_gjk_mixed_r<kRefineBlock, MESH><<<grid_for(n, (int)per), kRefineBlock, 0, stream>>>(
         store, i1, i2, order, n, (int)per, n_dev, opt, hand, o, lists);
     rc = check_launch("d3d_gjk_distance (mixed, refinement pass)");
@@ -872,11 +872,11 @@ int launch_mixed(const d3d_store& store, const int32_t* i1, const int32_t* i2, c
         set_error("d3d_gjk_distance (mixed, FP64 loop): %s", cudaGetErrorString(e));
         return D3D_ERR_CUDA;
     }
-    k_gjk_mixed_b<kLoopPool, MESH><<<persistent_blocks(kb, kLoopPool, n * kLoopPool, 0, smem), kLoopPool, smem, stream>>>(
+    k_gjk_mixed_b<kLoopPool, MESH><<<persistent_blocks(kb, kLoopPool, launch_items(n * kLoopPool, n / 4), 0, smem), kLoopPool, smem, stream>>>(
         store, i1, i2, opt, hand, o, lists);
     rc = check_launch("d3d_gjk_distance (mixed, FP64 loop)");
     if (rc) return rc;
-    k_gjk_mixed_end<<<persistent_blocks((const void*)k_gjk_mixed_end, 128, 32 * n), 128, 0, stream>>>(opt, o, lists);
+    k_gjk_mixed_end<<<persistent_blocks((const void*)k_gjk_mixed_end, 128, launch_items(32 * n, n)), 128, 0, stream>>>(opt, o, lists);
     return check_launch("d3d_gjk_distance (mixed, end pass)");
 }
 

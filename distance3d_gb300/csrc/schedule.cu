@@ -101,6 +101,14 @@ int persistent_blocks(const void* kernel, int block, int64_t work_items, int max
     return (int)(b > 0 ? b : 1);
 }
 
+namespace {
+thread_local bool t_shared_gpu = false;
+}
+
+SharedGpu::SharedGpu(bool on) : before_(t_shared_gpu) { t_shared_gpu = on; }
+SharedGpu::~SharedGpu() { t_shared_gpu = before_; }
+bool shared_gpu() { return t_shared_gpu; }
+
 d3d_tuning tuning() {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     return g_tuning;

@@ -20,6 +20,25 @@ void scratch_free(void* p, cudaStream_t stream);
 // max_per_sm if > 0) x SMs, capped by the work.
 int persistent_blocks(const void* kernel, int block, int64_t work_items, int max_per_sm = 0, int smem = 0);
 
+// While one lives, this thread's launches are for batches that run beside
+// others on the GPU: a small batch then takes the fewest blocks that hold its
+// pairs instead of the whole GPU, which would finish it sooner and the batches
+// beside it later.
+class SharedGpu {
+public:
+    explicit SharedGpu(bool on);
+    ~SharedGpu();
+    SharedGpu(const SharedGpu&) = delete;
+    SharedGpu& operator=(const SharedGpu&) = delete;
+
+private:
+    bool before_;
+};
+bool shared_gpu();
+
+// Work items to size a small batch's launch by: `alone` or, beside other batches, `dense`.
+inline int64_t launch_items(int64_t alone, int64_t dense) { return shared_gpu() ? dense : alone; }
+
 // The current launch parameters (d3d_set_tuning / d3d_autotune).
 d3d_tuning tuning();
 

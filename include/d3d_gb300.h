@@ -305,12 +305,11 @@ int d3d_chain_contacts(const double* dist, int64_t n_configs, const int32_t* pai
                        uint8_t* contacts, void* stream);
 
 /* Launch parameters of the batch kernels (process-wide, per library load).
- * gjk_block: threads per block of the GJK kernels (64, 128 or 256; the
- * plain FP64 GJK, whose blocks solve their simplices together, runs 128 for
- * 256);
- * gjk_warps_per_sm: resident warps per SM of their persistent grids (0: as
- * many as fit); epa_warps: pairs (warps) per block of the warp EPA (2, 4 or
- * 8); sort_min: batches of at least this many pairs are sorted by collider
+ * gjk_block: threads per block of the mixed GJK's FP32 phase (64, 128 or 256;
+ * the FP64 kernels' pools have their own size);
+ * gjk_warps_per_sm: resident warps per SM of the persistent GJK grids (0: as
+ * many as fit); epa_warps: warps per block of the mixed EPA (2, 4 or 8);
+ * sort_min: batches of at least this many pairs are sorted by collider
  * types before GJK (larger than any batch: never). */
 typedef struct {
     int32_t gjk_block;
