@@ -1370,7 +1370,10 @@ int launch_segments(const d3d_store& store, const int32_t* i1, const int32_t* i2
 // lanes, us: 64 faces (2,824 bytes): 900 pairs 101, 125, 142; 6,667 pairs 156,
 // 179, 194; 13,333 pairs 376, 233, 241; 33,333 pairs 611, 436, 365.  256 faces
 // (4,528 bytes): 6,667 pairs 212, 247, 279; 13,333 pairs 450, 284, 307;
-// 310,000 pairs 4,939, 3,357, 3,736.
+// 310,000 pairs 4,939, 3,357, 3,736.  Beside other batches (shared_gpu) the form
+// of a whole warp is left out, and the grid holds a quarter of n, about the
+// pairs that intersect (16 server slots: 51.3 M pairs/s; an eighth 49.2, all of
+// n 45.5).
 template <int WARPS, bool MESH>
 int launch_search(const d3d_store& store, const int32_t* i1, const int32_t* i2, const int32_t* list, int64_t n,
                   const unsigned long long* n_dev, unsigned long long* cursor, const double* simplex,
