@@ -893,11 +893,25 @@ int launch_mixed(const d3d_store& store, const int32_t* i1, const int32_t* i2, c
                                       per_sm, stream);
 }
 
+// lanes of phase A's full grid (phase_a_min_blocks)
+static int64_t phase_a_lanes() {
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return 512 * (int64_t)sms;
+}
+
 int gjk_mixed_run(const d3d_store& store, const int32_t* i1, const int32_t* i2, int64_t n, const int64_t* n_dev,
                   const d3d_gjk_options& opt, const DistanceOut& o, void* scratch, cudaStream_t stream,
                   const int32_t** sorted) {
     const d3d_tuning t = tuning();
-    const bool sched = n >= t.sort_min;
+    // Sorted by type only where phase A fills the GPU (or runs beside other
+    // batches): in a spread grid R, B and the EPA list their work by type
+    // anyway, phase A's warps hold few lanes, and sorting puts the long pairs
+    // into the same warps.  Sorted -> unsorted, us: six types 10,000 pairs 487
+    // -> 413, 65,536 925 -> 726, 77,000 963 -> 793, 262,144 1,522 -> 1,605; ten
+    // types 20,011 569 -> 538, 77,000 895 -> 818, 90,000 958 -> 1,047.
+    const bool sched = n >= t.sort_min && (shared_gpu() || n >= phase_a_lanes());
     const size_t c = (size_t)n;
     const size_t order_bytes = up(sizeof(int32_t) * c);
     const size_t temp_bytes = pair_order_temp_bytes(n);
