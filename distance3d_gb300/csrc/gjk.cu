@@ -74,7 +74,13 @@ int launch_pool(const d3d_store& store, const int32_t* i1, const int32_t* i2, co
 
 int intersect_part(const d3d_store& store, const int32_t* i1, const int32_t* i2, int64_t n, double tolerance,
                    int32_t max_iterations, int8_t* hit, int8_t* status, cudaStream_t stream) {
-    const bool sched = n >= tuning().sort_min;
+    // sorted by type only above what the pools hold at once: these searches are short, and a pool
+    // lists its supports by type itself.  Sorted -> unsorted, us: six types 5,000 pairs 171 -> 133,
+    // 65,536 282 -> 241; ten types 244 -> 238, 457 -> 427, 262,144 911 -> 986.
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const bool sched = n >= tuning().sort_min && n >= 2 * kPool * (int64_t)sms;
     void* block = nullptr;
     int rc = scratch_alloc(&block, sched ? gjk_f64_scratch_bytes(n) : 256, stream);
     if (rc) return rc;
