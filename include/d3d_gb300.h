@@ -310,7 +310,8 @@ int d3d_chain_contacts(const double* dist, int64_t n_configs, const int32_t* pai
  * gjk_warps_per_sm: resident warps per SM of the persistent GJK grids (0: as
  * many as fit); epa_warps: warps per block of the mixed EPA (2, 4 or 8);
  * sort_min: batches of at least this many pairs are sorted by collider
- * types before GJK (larger than any batch: never). */
+ * types before GJK (larger than any batch: never; the mixed GJK and the
+ * intersection test leave batches below a full grid unsorted). */
 typedef struct {
     int32_t gjk_block;
     int32_t gjk_warps_per_sm;
