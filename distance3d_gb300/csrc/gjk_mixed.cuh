@@ -264,8 +264,6 @@ struct __align__(16) Handoff {
     float4 d[4];
 };
 
-__device__ __forceinline__ int handoff_outcome(const Handoff& h) { return __float_as_int(h.v.w) & 0xff; }
-__device__ __forceinline__ int handoff_rows(const Handoff& h) { return (__float_as_int(h.v.w) >> 8) & 0xff; }
 __device__ __forceinline__ int handoff_iters(float4 v) { return (__float_as_int(v.w) >> 16) & 0xffff; }
 // the vertex collider k (0: i1, 1: i2) of a row took, -1 if none
 __device__ __forceinline__ int handoff_vertex(float4 d, int k) {

@@ -242,8 +242,8 @@ __device__ __forceinline__ void lane_support(M& m, const d3d_store& st, int e) {
     m.put_support(s, side, support(c, st, d));
 }
 
-// gjk_step_end (distance) or the rest of gjk_intersection_loop's iteration,
-// for slot s and the result of its solve; ysq(r) is |Y|^2 of place r.  Returns
+// gjk_step_end (distance) or the rest of the intersection test's iteration
+// (gjk_intersection_jolt, _gjk_jolt.py:29-135), for slot s and the result of its solve; ysq(r) is |Y|^2 of place r.  Returns
 // the intersection form's outcome, -1 while it runs.
 template <int S, int PQ, typename Ysq>
 __device__ __forceinline__ int finish_step(Mem<S, PQ>& m, int s, bool closer, d3 nv, double nl, int set, double tol_sq,

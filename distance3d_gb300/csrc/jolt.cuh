@@ -627,49 +627,4 @@ __device__ __forceinline__ void gjk_end(const GjkLoop<T, Rows>& g, T sanity, con
     out.b = b;
 }
 
-// The rest of the loop for one pair, from the state gjk_begin (and any
-// starting simplex) left in g: gjk_distance_jolt (_gjk_jolt.py:138-221).
-template <typename T, typename Sup = ExactSupport, bool GAP = false, bool SCALED = false, typename Rows>
-__device__ __forceinline__ void gjk_run(GjkLoop<T, Rows>& g, const d3d_store& st, int a, int b, T tol_sq, T max_d2,
-                                        T sanity, int max_iter, const JoltEps<T>& E, GjkResult<T>& out,
-                                        T rel_gap = T(0), T abs_gap2 = T(0)) {
-    while (!gjk_step<T, Sup, GAP>(g, st, a, b, tol_sq, max_d2, max_iter, E, rel_gap, abs_gap2)) {
-    }
-    gjk_end<T, SCALED>(g, sanity, E, out);
-}
-
-// gjk_intersection_jolt, _gjk_jolt.py:29-135.  Returns 1 on intersection.
-template <typename T, typename Sup = ExactSupport>
-__device__ __forceinline__ int gjk_intersection_loop(const d3d_store& st, int a, int b, T tol_sq, int max_iter,
-                                                     const JoltEps<T>& E, int& status) {
-    Simplex<T> S;
-    simplex_clear(S);
-    T prev = maxf<T>();
-    V3<T> dir = mk(T(1), T(0), T(0));
-    status = D3D_STATUS_OK;
-    for (int it = 1;; ++it) {
-        if (it > max_iter) {
-            status = D3D_STATUS_MAX_ITER;
-            return 0;
-        }
-        V3<T> p, q;
-        pair_supports<T, Sup>(st, a, b, dir, p, q);
-        V3<T> w = p - q;
-        if (dot(dir, w) < -E.conv) return 0;
-        simplex_push(S, w, p, q);
-        V3<T> nv;
-        T vl;
-        int set;
-        if (!closest_to_origin(S, prev, E, nv, vl, set)) return 0;
-        dir = nv;
-        if (set == 15) return 1;
-        if (vl <= tol_sq) return 1;
-        if (vl <= E.isect * max_y_len_sq(S)) return 1;
-        dir = -dir;
-        if (prev - vl <= E.conv * prev) return 0;
-        prev = vl;
-        simplex_compact<T, false>(S, set);
-    }
-}
-
 }  // namespace d3d
