@@ -106,15 +106,17 @@ __global__ void __launch_bounds__(BLOCK, phase_a_min_blocks<BLOCK>()) k_gjk_mixe
     int64_t pid = 0;
     int a = 0, b = 0;
     const long long lanes = spread_lanes(n, BLOCK);
-    bool have = false, bad = false, exhausted = (int)(threadIdx.x & 31) >= lanes;
+    bool have = false, bad = false;
+    int part = lane_part((int)(threadIdx.x & 31) < lanes);
     WarpChunk chunk;
     while (true) {
         __syncwarp();
-        const bool want = !have && !exhausted;
+        part = next_part(part, lists.ctr + kCurA, n);
+        const bool want = !have && part == 0;
         const long long slot = fetch_slot_chunked(lists.ctr + kCurA, want, chunk, kAll, kChunk, 0);
         if (want) {
             if (slot >= n) {
-                exhausted = true;
+                part = kOut;
             } else {
                 pid = order ? order[slot] : slot;
                 a = i1[pid];
@@ -531,7 +533,7 @@ __global__ void __launch_bounds__(S, 3) k_gjk_mixed_b(d3d_store st, const int32_
     const double tol_sq = opt.tolerance * opt.tolerance;
     const long long share = (n + gridDim.x - 1) / gridDim.x;
     const long long split = share < S ? 0 : n;
-    bool exhausted = t >= share;
+    int part = lane_part(t < share);
     WarpChunk chunk;
     m.meta[t] = 0;
     if (t < kBins) m.cnt[0][t] = m.cnt[1][t] = 0;
@@ -541,11 +543,12 @@ __global__ void __launch_bounds__(S, 3) k_gjk_mixed_b(d3d_store st, const int32_
     for (int par = 0;; par ^= 1) {
         // ---- free slots take new pairs
         int state = pool::meta_state(m.meta[t]);
-        const bool want = state == pool::kFree && !exhausted;
+        part = next_part(part, lists.ctr + kCurB, n);
+        const bool want = state == pool::kFree && part == 0;
         const long long slot = fetch_slot_chunked(lists.ctr + kCurB, want, chunk, kAll, kChunk, split);
         if (want) {
             if (slot >= n) {
-                exhausted = true;
+                part = kOut;
             } else {
                 const int pid = lists.run[slot];
                 const EndRecord& rec = lists.records[pid];
@@ -590,7 +593,7 @@ __global__ void __launch_bounds__(S, 3) k_gjk_mixed_b(d3d_store st, const int32_
             if (ln == leader && bin >= 0) base = atomicAdd(&m.cnt[par][bin], __popc(same));
             pos[k] = __shfl_sync(kAll, base, leader) + __popc(same & ((1u << ln) - 1u));
         }
-        if (!__syncthreads_or(state != pool::kFree || !exhausted)) break;
+        if (!__syncthreads_or(state != pool::kFree || part == 0)) break;
         const Chunks ch = chunks_of(m.cnt[par], kBins, (ln >> 1) == D3D_HULL ? pool::kHullChunk : 32);
 #pragma unroll
         for (int k = 0; k < 2; ++k) {

@@ -649,7 +649,7 @@ __global__ void __launch_bounds__(S, 512 / S) k_gjk_pool(d3d_store st, const int
     // a batch that does not fill every block is spread evenly over them
     const long long share = (n + gridDim.x - 1) / gridDim.x;
     const long long split = share < S ? 0 : n;
-    bool exhausted = t >= share;
+    int part = lane_part(t < share);
     WarpChunk chunk;
     m.meta[t] = 0;
     if (t < kBins) m.cnt[0][t] = m.cnt[1][t] = 0;
@@ -659,11 +659,12 @@ __global__ void __launch_bounds__(S, 512 / S) k_gjk_pool(d3d_store st, const int
     for (int par = 0;; par ^= 1) {
         // ---- free slots take new pairs
         int state = meta_state(m.meta[t]);
-        const bool want = state == kFree && !exhausted;
+        part = next_part(part, cursor, n);
+        const bool want = state == kFree && part == 0;
         const long long slot = fetch_slot_chunked(cursor, want, chunk, kAll, kFetch, split);
         if (want) {
             if (slot >= n) {
-                exhausted = true;
+                part = kOut;
             } else {
                 const int pid = order ? order[slot] : (int)slot;
                 const int a = i1[pid], b = i2[pid];
@@ -704,7 +705,7 @@ __global__ void __launch_bounds__(S, 512 / S) k_gjk_pool(d3d_store st, const int
             if (ln == leader && bin >= 0) base = atomicAdd(&m.cnt[par][bin], __popc(same));
             pos[k] = __shfl_sync(kAll, base, leader) + __popc(same & ((1u << ln) - 1u));
         }
-        if (!__syncthreads_or(state != kFree || !exhausted)) break;
+        if (!__syncthreads_or(state != kFree || part == 0)) break;
         // bin ln of the list: its first task and first chunk; the finished pairs wait until they
         // fill a warp, or no pair is left to iterate
         const int size = (ln >> 1) == D3D_HULL ? kHullChunk : 32;

@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kSlots, 2) k_mpr(d3d_store st, const int32_t* 
     // a batch that does not fill every block is spread evenly over them
     const long long share = (n + gridDim.x - 1) / gridDim.x;
     const long long split = share < kSlots ? 0 : n;
-    bool exhausted = t >= share;
+    int part = lane_part(t < share);
     WarpChunk chunk;
     m.meta[t] = 0;
     if (t < kBins) m.cnt[0][t] = m.cnt[1][t] = 0;
@@ -125,11 +125,12 @@ __global__ void __launch_bounds__(kSlots, 2) k_mpr(d3d_store st, const int32_t* 
     for (int par = 0;; par ^= 1) {
         // ---- free slots take new pairs
         int meta = m.meta[t];
-        const bool want = (meta & 3) == kFree && !exhausted;
+        part = next_part(part, cursor, n);
+        const bool want = (meta & 3) == kFree && part == 0;
         const long long slot = fetch_slot_chunked(cursor, want, chunk, kAll, 32, split);
         if (want) {
             if (slot >= n) {
-                exhausted = true;
+                part = kOut;
             } else {
                 const int pid = order ? order[slot] : (int)slot;
                 const int c[2] = {i1[pid], i2[pid]};
@@ -165,7 +166,7 @@ __global__ void __launch_bounds__(kSlots, 2) k_mpr(d3d_store st, const int32_t* 
             if (ln == leader && bin[k] >= 0) base = atomicAdd(&m.cnt[par][bin[k]], __popc(same));
             pos[k] = __shfl_sync(kAll, base, leader) + __popc(same & ((1u << ln) - 1u));
         }
-        const int running = __syncthreads_or((state != kFree || !exhausted ? 1 : 0) | (state == kLive ? 2 : 0));
+        const int running = __syncthreads_or((state != kFree || part == 0 ? 1 : 0) | (state == kLive ? 2 : 0));
         if (!running) break;
         // the finished pairs wait until they fill a warp, or no pair is left to iterate
         const bool ends = m.cnt[par][kEndBin] >= 32 || !(running & 2);
