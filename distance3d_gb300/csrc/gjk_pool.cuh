@@ -629,9 +629,24 @@ __device__ __forceinline__ void solve_wide(Mem<S, PQ>& m, int s, double tol_sq, 
                 hits, status);
 }
 
+// The pairs of a batch dealt to the blocks in runs of 1 << run: the lanes that
+// want one take the block's next, counted in *dealt (shared memory).
+__device__ __forceinline__ unsigned dealt_slot(unsigned* dealt, bool want, int run) {
+    const unsigned w = __ballot_sync(kAll, want);
+    if (!w) return 0u;
+    const int ln = threadIdx.x & 31, leader = __ffs(w) - 1;
+    unsigned x = 0;
+    if (ln == leader) x = atomicAdd(dealt, (unsigned)__popc(w));
+    x = __shfl_sync(kAll, x, leader) + __popc(w & ((1u << ln) - 1u));
+    return ((x >> run) * gridDim.x + blockIdx.x << run) | (x & ((1u << run) - 1u));
+}
+
 // The FP64 GJK distance (PQ = 4) or intersection test (PQ = 1) of the pairs
 // order[k] (or k), k < n (or *n_dev): see the top of this file.  S threads
-// and pairs per block.
+// and pairs per block.  The distances' blocks claim pairs from *cursor.  The
+// intersection test takes no memory but its arguments (null order, n_dev and
+// cursor): the pairs are dealt to the blocks in input order, and a block counts
+// its own in shared memory.
 template <int S, int PQ>
 __global__ void __launch_bounds__(S, 512 / S) k_gjk_pool(d3d_store st, const int32_t* __restrict__ i1,
                                                          const int32_t* __restrict__ i2,
@@ -649,8 +664,10 @@ __global__ void __launch_bounds__(S, 512 / S) k_gjk_pool(d3d_store st, const int
     // a batch that does not fill every block is spread evenly over them
     const long long share = (n + gridDim.x - 1) / gridDim.x;
     const long long split = share < S ? 0 : n;
-    int part = lane_part(t < share);
+    int part = kDistance ? lane_part(t < share) : (t < share ? 0 : kOut);
     WarpChunk chunk;
+    __shared__ unsigned dealt;
+    if (!kDistance && t == 0) dealt = 0u;
     m.meta[t] = 0;
     if (t < kBins) m.cnt[0][t] = m.cnt[1][t] = 0;
     if (t < 4) m.scnt[0][t] = m.scnt[1][t] = m.next[t >> 1][t & 1] = 0;
@@ -659,9 +676,10 @@ __global__ void __launch_bounds__(S, 512 / S) k_gjk_pool(d3d_store st, const int
     for (int par = 0;; par ^= 1) {
         // ---- free slots take new pairs
         int state = meta_state(m.meta[t]);
-        part = next_part(part, cursor, n);
+        if (kDistance) part = next_part(part, cursor, n);
         const bool want = state == kFree && part == 0;
-        const long long slot = fetch_slot_chunked(cursor, want, chunk, kAll, kFetch, split);
+        const long long slot = kDistance ? fetch_slot_chunked(cursor, want, chunk, kAll, kFetch, split)
+                                         : (long long)dealt_slot(&dealt, want, share < S ? 0 : 5);
         if (want) {
             if (slot >= n) {
                 part = kOut;

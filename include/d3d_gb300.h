@@ -199,7 +199,8 @@ int d3d_gjk_distance_cached(const d3d_store* store, const int32_t* i1, const int
 
 /* Batched Jolt GJK intersection test: hit[k] = 1 if the pair intersects.
  * Replaces gjk.gjk_intersection / gjk_intersection_jolt, _gjk_jolt.py:29-135
- * (alias gjk/__init__.py:28). */
+ * (alias gjk/__init__.py:28).  Runs in input order; allocates nothing, and a
+ * captured call holds one kernel node. */
 int d3d_gjk_intersection(const d3d_store* store, const int32_t* i1, const int32_t* i2,
                          int64_t n, double tolerance, int32_t max_iterations, int8_t* hit,
                          int8_t* status, void* stream);
@@ -310,8 +311,8 @@ int d3d_chain_contacts(const double* dist, int64_t n_configs, const int32_t* pai
  * gjk_warps_per_sm: resident warps per SM of the persistent GJK grids (0: as
  * many as fit); epa_warps: warps per block of the mixed EPA (2, 4 or 8);
  * sort_min: batches of at least this many pairs are sorted by collider
- * types before GJK (larger than any batch: never; the mixed GJK and the
- * intersection test leave batches below a full grid unsorted). */
+ * types before GJK (larger than any batch: never; the mixed GJK leaves batches
+ * below a full grid unsorted). */
 typedef struct {
     int32_t gjk_block;
     int32_t gjk_warps_per_sm;
