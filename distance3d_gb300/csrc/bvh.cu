@@ -171,20 +171,40 @@ __device__ __forceinline__ uint64_t spread21(uint64_t v) {
     return v;
 }
 
-// The scaling is FP32 (after an FP64 subtraction): the codes only shape the tree.
+// 21 bits of the center c on an axis of `least` and extent `ext`, in FP64.
+__device__ __noinline__ uint64_t axis_code(double c, double least, double ext) {
+    const double x = ext > 0.0 ? (c - least) / ext * 2097152.0 : 0.0;
+    return (x != x || x <= 0.0) ? 0ull : (x >= 2097151.0 ? 2097151ull : (uint64_t)x);
+}
+
+// axis_code's value without its division, bound by the FP64 pipe: 2^52 + (c -
+// least) * (2^52 / ext) holds the code in the upper 21 bits of its mantissa and
+// its fraction in the lower 31, a few units off axis_code's at most.  Where those
+// could carry into the code, and where the sum is not in [2^52, 2^53) (a NaN, an
+// extent out of range, the last center), axis_code decides.  Build of 200,003
+// boxes with the division 240 us, without 230 (scaled in FP32 it was 232).
 __global__ void k_morton(const double* __restrict__ aabbs, int64_t n, const unsigned long long* __restrict__ bounds,
                          uint64_t* __restrict__ keys, int32_t* __restrict__ vals) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ double least[3], ext[3], scale[3];
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    double lo[3] = {}, hi[3] = {};
+    if (i < n) load_box(aabbs, i, lo, hi);
+    if (threadIdx.x < 3) {
+        const int k = threadIdx.x;
+        least[k] = from_key(~bounds[k]);
+        ext[k] = from_key(bounds[3 + k]) - least[k];
+        scale[k] = 0x1p52 / ext[k];
+    }
+    __syncthreads();
     if (i >= n) return;
-    double lo[3], hi[3];
-    load_box(aabbs, i, lo, hi);
     uint64_t q[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const double least = from_key(~bounds[k]);
-        const float ext = (float)(from_key(bounds[3 + k]) - least);
-        const float x = (float)(0.5 * (lo[k] + hi[k]) - least) * (2097152.f / ext);
-        q[k] = !(x > 0.f) ? 0ull : (x >= 2097151.f ? 2097151ull : (uint64_t)x);
+        const double c = 0.5 * (lo[k] + hi[k]);
+        const uint64_t b = (uint64_t)__double_as_longlong(fma(c - least[k], scale[k], 0x1p52));
+        const uint32_t rest = (uint32_t)b & 0x7fffffffu;
+        const bool sure = (b >> 52) == 0x433u && rest - 8u < 0x7fffffffu - 16u;
+        q[k] = sure ? (b >> 31) & 0x1fffffu : axis_code(c, least[k], ext[k]);
     }
     keys[i] = (spread21(q[0]) << 2) | (spread21(q[1]) << 1) | spread21(q[2]);
     vals[i] = (int32_t)i;
