@@ -386,10 +386,7 @@ def serve_report(store, i1_np, i2_np, seconds, seed=7, capacity=4096, slots=16, 
     from distance3d_gb300.tune import autotune, get_tuning, set_tuning
     rng = np.random.default_rng(seed)
     mean_size = float(request_sizes(np.random.default_rng(seed + 1), 200000).mean())
-    # the launch parameters for the server's saturated regime, every slot's
-    # batch in flight: tuned on capacity * slots pairs (restored after)
     before = get_tuning()
-    tuned = autotune(store, i1_np[:capacity * slots], i2_np[:capacity * slots], epa_kw=EPA_KW)
 
     def trace(count):
         sizes = request_sizes(rng, count)
@@ -398,8 +395,13 @@ def serve_report(store, i1_np, i2_np, seconds, seed=7, capacity=4096, slots=16, 
 
     out = {"request_pairs": {"median": 2000, "clip": [1, 50000], "mean": mean_size},
            "latency": "arrival to results in host memory", "server": "native (d3d_server), CUDA graphs",
-           "capacity": capacity, "slots": slots, "tuning": tuned}
+           "capacity": capacity, "slots": slots, "tuning": {}}
     for precision in ("mixed", "fp64"):
+        # the launch parameters for the server's saturated regime, every slot's
+        # batch in flight: tuned on as many batches side by side
+        set_tuning(**before)
+        out["tuning"][precision] = autotune(store, i1_np[:capacity * slots], i2_np[:capacity * slots],
+                                            precision=precision, epa_kw=EPA_KW, batches=slots)
         # the worker thread asks for SCHED_FIFO priority 1 (a thread that sleeps between passes), so
         # that other threads on the host do not delay its launches; the stats say whether it got it
         srv = NativeCollisionServer(store, capacity=capacity, slots=slots, precision=precision, epa_kw=EPA_KW,

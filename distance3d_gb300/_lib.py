@@ -108,6 +108,8 @@ SIGNATURES = [
     ("d3d_chain_contacts", c_int, [c_void_p, c_int64, c_void_p, c_int64, c_int32, c_void_p, c_void_p]),
     ("d3d_get_tuning", c_int, [ctypes.POINTER(Tuning)]),
     ("d3d_set_tuning", c_int, [ctypes.POINTER(Tuning)]),
+    ("d3d_autotune_batches", c_int, [_SP, c_void_p, c_void_p, c_int64, c_int32, ctypes.POINTER(GjkOptions),
+                                     ctypes.POINTER(EpaOptions), ctypes.POINTER(Tuning), c_void_p]),
     ("d3d_autotune", c_int, [_SP, c_void_p, c_void_p, c_int64, ctypes.POINTER(GjkOptions), ctypes.POINTER(EpaOptions),
                              ctypes.POINTER(Tuning), c_void_p]),
     ("d3d_server_create", c_int, [_SP, ctypes.POINTER(GjkOptions), ctypes.POINTER(EpaOptions),

@@ -33,6 +33,9 @@ int epa_mixed_launch(const d3d_store& store, const int32_t* i1, const int32_t* i
 // FP64 form takes neither), and a second kernel then computes the pairs' FP64
 // depths along those normals, one pair per thread.
 bool epa_warp_supported(const d3d_epa_options& o, bool fp64 = false);
+// Warps per block the form launches under tuning t, as tuned or fewer if their
+// polytopes do not fit in one block.
+int epa_warp_count(const d3d_tuning& t, const d3d_epa_options& o, bool fp64);
 int epa_warp_launch(const d3d_store& store, const int32_t* i1, const int32_t* i2, const int32_t* list, int64_t n,
                     const unsigned long long* n_dev, unsigned long long* cursor, const double* simplex,
                     const d3d_epa_options& o, double* mtv, int8_t* status, int32_t* n_faces, double* faces,

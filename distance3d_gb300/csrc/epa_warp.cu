@@ -1449,15 +1449,19 @@ bool epa_warp_supported(const d3d_epa_options& o, bool fp64) {
     return (int64_t)bytes * 2 <= kSmemPerBlock;
 }
 
+int epa_warp_count(const d3d_tuning& t, const d3d_epa_options& o, bool fp64) {
+    const int64_t bytes = fp64 ? layout_for<double>(o).bytes : layout_for<float>(o).bytes;
+    int w = t.epa_warps;
+    while (w > 2 && bytes * w > kSmemPerBlock) w /= 2;
+    return w;
+}
+
 int epa_warp_launch(const d3d_store& store, const int32_t* i1, const int32_t* i2, const int32_t* list, int64_t n,
                     const unsigned long long* n_dev, unsigned long long* cursor, const double* simplex,
                     const d3d_epa_options& o, double* mtv, int8_t* status, int32_t* n_faces, double* faces,
                     int32_t* fallback, unsigned long long* n_fallback, cudaStream_t stream, bool fp64,
                     int32_t* refine, unsigned long long* n_refine) {
-    // pairs per block as tuned, fewer if their polytopes do not fit in one block
-    const int64_t bytes = fp64 ? layout_for<double>(o).bytes : layout_for<float>(o).bytes;
-    int w = tuning().epa_warps;
-    while (w > 2 && bytes * w > kSmemPerBlock) w /= 2;
+    const int w = epa_warp_count(tuning(), o, fp64);
 #define D3D_WARP_LAUNCH(T, W)                                                                                      \
     return launch_warp<T, W>(store, i1, i2, list, n, n_dev, cursor, simplex, o, mtv, status, n_faces, faces, fallback, \
                              n_fallback, refine, n_refine, stream)

@@ -53,6 +53,13 @@ __global__ void __launch_bounds__(128) k_gjk_distance_f64_cached(d3d_store s, co
 constexpr int kPool = 256;
 
 template <int PQ>
+int pool_blocks(const d3d_tuning& t, int64_t n) {
+    // a block per pair for the smallest batches: their pairs run side by side
+    return persistent_blocks((const void*)pool::k_gjk_pool<kPool, PQ>, kPool, launch_items(n * kPool, n),
+                             blocks_per_sm(t, kPool), (int)sizeof(pool::Mem<kPool, PQ>));
+}
+
+template <int PQ>
 int launch_pool(const d3d_store& store, const int32_t* i1, const int32_t* i2, const int32_t* order, int64_t n,
                 const unsigned long long* n_dev, unsigned long long* cursor, const d3d_gjk_options& opt,
                 const DistanceOut& o, int8_t* hits, cudaStream_t stream) {
@@ -66,9 +73,7 @@ int launch_pool(const d3d_store& store, const int32_t* i1, const int32_t* i2, co
         set_error("FP64 GJK: %s", cudaGetErrorString(e));
         return D3D_ERR_CUDA;
     }
-    // a block per pair for the smallest batches: their pairs run side by side
-    const int blocks = persistent_blocks(fn, kPool, launch_items(n * kPool, n), blocks_per_sm(tuning(), kPool), smem);
-    pool::k_gjk_pool<kPool, PQ><<<blocks, kPool, smem, stream>>>(store, i1, i2, order, n, n_dev, cursor, opt, o, hits);
+    pool::k_gjk_pool<kPool, PQ><<<pool_blocks<PQ>(tuning(), n), kPool, smem, stream>>>(store, i1, i2, order, n, n_dev, cursor, opt, o, hits);
     return check_launch(PQ == 4 ? "d3d_gjk_distance" : "d3d_gjk_intersection");
 }
 
@@ -102,6 +107,8 @@ extern "C" int d3d_gjk_distance(const d3d_store* store, const int32_t* i1, const
 }
 
 namespace d3d {
+
+GjkLaunch gjk_f64_launch(const d3d_tuning& t, int64_t n) { return {0, 0, pool_blocks<4>(t, n), n >= t.sort_min}; }
 
 size_t gjk_f64_scratch_bytes(int64_t capacity) {
     return 256 + ((sizeof(int32_t) * (size_t)capacity + 255) & ~size_t(255)) + pair_order_temp_bytes(capacity);

@@ -15,6 +15,20 @@ int launch_gjk_f64(const d3d_store& store, const int32_t* i1, const int32_t* i2,
                    const unsigned long long* n_dev, unsigned long long* cursor, const d3d_gjk_options& opt,
                    const DistanceOut& o, cudaStream_t stream);
 
+// What a batch of n pairs launches under tuning t (the tuner leaves out
+// candidates that launch the same).
+struct GjkLaunch {
+    int block;         // threads per block of the mixed form's FP32 phase, and its blocks; 0: none
+    int blocks;
+    int pool_blocks;   // of the FP64 pool
+    bool sorted;       // by type
+    bool operator==(const GjkLaunch& o) const {
+        return block == o.block && blocks == o.blocks && pool_blocks == o.pool_blocks && sorted == o.sorted;
+    }
+};
+GjkLaunch gjk_f64_launch(const d3d_tuning& t, int64_t n);
+GjkLaunch gjk_mixed_launch(const d3d_store& store, const d3d_tuning& t, int64_t n);
+
 // The mixed form on caller scratch (gjk_mixed_scratch_bytes(n)); with n_dev,
 // the pair count is *n_dev <= n, read on the device, and the launches depend
 // on n only (a CUDA graph can hold them).  `sorted`, if not null, receives the

@@ -832,12 +832,17 @@ constexpr int kLoopPool = 128;
 constexpr int kRefineBlock = 128;
 
 template <int BLOCK, bool MESH>
+int phase_a_blocks(int64_t n, int per_sm) {
+    // alone: down to a pair per warp
+    return persistent_blocks((const void*)k_gjk_mixed_a<BLOCK, MESH>, BLOCK, launch_items(32 * n, n), per_sm);
+}
+
+template <int BLOCK, bool MESH>
 int launch_mixed(const d3d_store& store, const int32_t* i1, const int32_t* i2, const int32_t* order, int64_t n,
                  const int64_t* n_dev, const d3d_gjk_options& opt, Handoff* hand, const DistanceOut& o,
                  const Lists& lists, void* select_temp, size_t select_bytes, int per_sm, cudaStream_t stream) {
     const float tol_sq = (float)(opt.tolerance * opt.tolerance);
-    const void* ka = (const void*)k_gjk_mixed_a<BLOCK, MESH>;
-    const int full = persistent_blocks(ka, BLOCK, launch_items(32 * n, n), per_sm);  // alone: down to a pair per warp
+    const int full = phase_a_blocks<BLOCK, MESH>(n, per_sm);
     if (shared_gpu() || n >= (int64_t)full * BLOCK)
         k_gjk_mixed_a<BLOCK, MESH><<<full, BLOCK, 0, stream>>>(store, i1, i2, order, n, n_dev, tol_sq,
                                                                (float)opt.max_distance_squared, opt.max_iterations,
@@ -896,25 +901,37 @@ int launch_mixed(const d3d_store& store, const int32_t* i1, const int32_t* i2, c
                                       per_sm, stream);
 }
 
-// lanes of phase A's full grid (phase_a_min_blocks)
-static int64_t phase_a_lanes() {
+// Sorted by type only where phase A fills the GPU (or runs beside other
+// batches): in a spread grid R, B and the EPA list their work by type
+// anyway, phase A's warps hold few lanes, and sorting puts the long pairs
+// into the same warps.  Sorted -> unsorted, us: six types 10,000 pairs 487
+// -> 413, 65,536 925 -> 726, 77,000 963 -> 793, 262,144 1,522 -> 1,605; ten
+// types 20,011 569 -> 538, 77,000 895 -> 818, 90,000 958 -> 1,047.
+static bool mixed_sorted(const d3d_tuning& t, int64_t n) {
+    if (shared_gpu()) return n >= t.sort_min;
     int dev = 0, sms = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return 512 * (int64_t)sms;
+    return n >= sort_from(t, 512 * (int64_t)sms);  // lanes of the full grid (phase_a_min_blocks)
+}
+
+template <bool MESH>
+static int phase_a_blocks(const d3d_tuning& t, int64_t n) {
+    if (t.gjk_block == 64) return phase_a_blocks<64, MESH>(n, blocks_per_sm(t, 64));
+    if (t.gjk_block == 256) return phase_a_blocks<256, MESH>(n, blocks_per_sm(t, 256));
+    return phase_a_blocks<128, MESH>(n, blocks_per_sm(t, 128));
+}
+
+GjkLaunch gjk_mixed_launch(const d3d_store& store, const d3d_tuning& t, int64_t n) {
+    const int blocks = store.n_links > 0 ? phase_a_blocks<true>(t, n) : phase_a_blocks<false>(t, n);
+    return {t.gjk_block, blocks, gjk_f64_launch(t, n).pool_blocks, mixed_sorted(t, n)};
 }
 
 int gjk_mixed_run(const d3d_store& store, const int32_t* i1, const int32_t* i2, int64_t n, const int64_t* n_dev,
                   const d3d_gjk_options& opt, const DistanceOut& o, void* scratch, cudaStream_t stream,
                   const int32_t** sorted) {
     const d3d_tuning t = tuning();
-    // Sorted by type only where phase A fills the GPU (or runs beside other
-    // batches): in a spread grid R, B and the EPA list their work by type
-    // anyway, phase A's warps hold few lanes, and sorting puts the long pairs
-    // into the same warps.  Sorted -> unsorted, us: six types 10,000 pairs 487
-    // -> 413, 65,536 925 -> 726, 77,000 963 -> 793, 262,144 1,522 -> 1,605; ten
-    // types 20,011 569 -> 538, 77,000 895 -> 818, 90,000 958 -> 1,047.
-    const bool sched = n >= t.sort_min && (shared_gpu() || n >= phase_a_lanes());
+    const bool sched = mixed_sorted(t, n);
     const size_t c = (size_t)n;
     const size_t order_bytes = up(sizeof(int32_t) * c);
     const size_t temp_bytes = pair_order_temp_bytes(n);

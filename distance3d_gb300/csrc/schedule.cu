@@ -19,7 +19,7 @@ cudaMemPool_t g_pool[kMaxDevices] = {};
 inline size_t align_up(size_t x) { return (x + 255) & ~size_t(255); }
 
 std::mutex g_tune_mu;
-d3d_tuning g_tuning = {128, 0, 4, 4096};
+d3d_tuning g_tuning = {128, 0, 4, d3d::kSortMin};
 
 // key = ((type1 * 10 + type2) << 4) | size class of the larger hull or mesh
 // (at most 99 * 16 + 15 < 2^11); slots at and beyond the device-side count (if given)

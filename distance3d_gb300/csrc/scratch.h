@@ -36,11 +36,25 @@ private:
 };
 bool shared_gpu();
 
+// A server of more slots than this, or the tuner for as many batches, launches
+// for a shared GPU.  A batch of 4,096 pairs alone on the whole GPU takes 0.57
+// ms instead of 0.77, but 16 slots of them run one after the other.  Peak M
+// pairs/s of 2,000-pair requests with / without: 16 slots 51.3 / 31.7 (FP64
+// 10.4 / 8.8), 8 slots 32.8 / 28.2, 4 slots 18.0 / 21.3 (FP64 5.3 / 4.8).
+constexpr size_t kAloneBatches = 4;
+
 // Work items to size a small batch's launch by: `alone` or, beside other batches, `dense`.
 inline int64_t launch_items(int64_t alone, int64_t dense) { return shared_gpu() ? dense : alone; }
 
 // The current launch parameters (d3d_set_tuning / d3d_autotune).
 d3d_tuning tuning();
+
+// Pairs from which on a batch is sorted by type: sort_min as it is set, and the
+// kernel's own rule (`measured`) above it while it has its first value.
+constexpr int32_t kSortMin = 4096;
+inline int64_t sort_from(const d3d_tuning& t, int64_t measured) {
+    return t.sort_min == kSortMin && measured > kSortMin ? measured : t.sort_min;
+}
 
 // blocks per SM for a GJK grid of `block` threads under tuning t (0: no cap)
 inline int blocks_per_sm(const d3d_tuning& t, int block) {

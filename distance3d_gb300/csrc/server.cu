@@ -113,15 +113,8 @@ int cuda_fail(d3d_server* s, cudaError_t e, const char* what) {
     return D3D_ERR_CUDA;
 }
 
-// Servers of more slots launch their batches for a GPU shared with the other
-// slots' (SharedGpu): a batch of 4,096 pairs alone on the whole GPU takes 0.57
-// ms instead of 0.77, but 16 slots of them run one after the other.  Peak M
-// pairs/s of 2,000-pair requests with / without: 16 slots 51.3 / 29.9 (FP64
-// 10.2 / 4.6), 8 slots 32.6 / 26.5, 4 slots 18.0 / 21.3 (FP64 5.3 / 3.9).
-constexpr size_t kAloneSlots = 4;
-
 int collide(d3d_server* s, Slot& sl, int64_t cap) {
-    const d3d::SharedGpu shared(s->slots.size() > kAloneSlots);
+    const d3d::SharedGpu shared(s->slots.size() > d3d::kAloneBatches);
     return d3d_collide(&s->store, sl.i1, sl.i2, cap, sl.n_dev, &s->gjk, &s->epa, (double*)sl.out[0],
                        (double*)sl.out[1], (double*)sl.out[2], (double*)sl.out[3], (int8_t*)sl.out[4],
                        (int8_t*)sl.out[5], (int32_t*)sl.out[6], (double*)sl.out[7], (int8_t*)sl.out[8],

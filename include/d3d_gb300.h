@@ -311,8 +311,10 @@ int d3d_chain_contacts(const double* dist, int64_t n_configs, const int32_t* pai
  * gjk_warps_per_sm: resident warps per SM of the persistent GJK grids (0: as
  * many as fit); epa_warps: warps per block of the mixed EPA (2, 4 or 8);
  * sort_min: batches of at least this many pairs are sorted by collider
- * types before GJK (larger than any batch: never; the mixed GJK leaves batches
- * below a full grid unsorted). */
+ * types before GJK and MPR (larger than any batch: never).  At its first
+ * value, 4096, the mixed GJK sorts from a full grid of its FP32 phase on (512
+ * pairs per SM), below which sorting costs more than it gives; any other value
+ * is taken as it is.  The intersection test never sorts. */
 typedef struct {
     int32_t gjk_block;
     int32_t gjk_warps_per_sm;
@@ -323,9 +325,15 @@ int d3d_get_tuning(d3d_tuning* out);
 int d3d_set_tuning(const d3d_tuning* tuning);
 /* Time candidate tunings on the given pairs (GJK distance and EPA, both in
  * options' precisions, on `stream`), set the fastest and return it in *out.
+ * A parameter that n pairs in these precisions do not read keeps its value,
+ * and the setting that was there stays unless another is 2 % faster.
  * Blocks until done. */
 int d3d_autotune(const d3d_store* store, const int32_t* i1, const int32_t* i2, int64_t n,
                  const d3d_gjk_options* gjk, const d3d_epa_options* epa, d3d_tuning* out, void* stream);
+/* The same for `batches` batches of n pairs each (i1, i2: batches x n pairs)
+ * that run side by side, as a server of as many slots launches them. */
+int d3d_autotune_batches(const d3d_store* store, const int32_t* i1, const int32_t* i2, int64_t n, int32_t batches,
+                         const d3d_gjk_options* gjk, const d3d_epa_options* epa, d3d_tuning* out, void* stream);
 
 /* Continuous-batching collision server over one resident store (no
  * counterpart in the reference, which answers one pair per call).  A worker
