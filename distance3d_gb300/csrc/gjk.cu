@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(128) k_gjk_distance_f64_cached(d3d_store s, co
     gjk_begin(g, dir, dot(dir, dir), DBL_MAX);
     int cache[2] = {mesh_cache[2 * k], mesh_cache[2 * k + 1]};
     const double tol_sq = opt.tolerance * opt.tolerance;
-    while (!gjk_step<double>(g, s, a, b, tol_sq, opt.max_distance_squared, opt.max_iterations, E, 0.0, 0.0, cache)) {
+    while (!gjk_step<double>(g, s, a, b, tol_sq, opt.max_distance_squared, opt.max_iterations, E, cache)) {
     }
     GjkResult<double> r;
     gjk_end(g, opt.sanity_check, E, r);

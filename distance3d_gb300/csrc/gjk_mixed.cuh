@@ -389,7 +389,7 @@ __device__ __forceinline__ int pa_step(PhaseALoop<Rows>& L, bool on, const d3d_s
     }
     L.v = L.dir;
     if (set == 15) return PA_TOUCHING;
-    simplex_compact<float, true>(L.S, set);
+    simplex_compact(L.S, set);
     if (L.vl <= tol_sq || L.vl <= E.isect * max_y_len_sq(L.S)) return PA_TOUCHING;
     L.dir = -L.dir;
     if (L.prev - L.vl <= E.conv * L.prev) return (L.vl == L.vl && L.vl <= FLT_MAX) ? PA_SEPARATED : PA_FAILED;

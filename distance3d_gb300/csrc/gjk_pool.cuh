@@ -23,7 +23,7 @@
 //   solve     tetrahedra sixteen per chunk: four lanes test the four planes of
 //             one, then the faces that see the origin, one per lane; triangles,
 //             segments and points one per lane; the solving lane also ends the
-//             iteration (gjk_step_end)
+//             iteration (finish_step)
 //
 // The simplex rows never move: a pair's four logical rows map to four places
 // through two bits each, so compaction is integer work; a row's place stays
@@ -242,7 +242,7 @@ __device__ __forceinline__ void lane_support(M& m, const d3d_store& st, int e) {
     m.put_support(s, side, support(c, st, d));
 }
 
-// gjk_step_end (distance) or the rest of the intersection test's iteration
+// The rest of gjk_step after its solve (distance) or the rest of the intersection test's iteration
 // (gjk_intersection_jolt, _gjk_jolt.py:29-135), for slot s and the result of its solve; ysq(r) is |Y|^2 of place r.  Returns
 // the intersection form's outcome, -1 while it runs.
 template <int S, int PQ, typename Ysq>
@@ -794,7 +794,7 @@ __global__ void __launch_bounds__(S, 512 / S) k_gjk_pool(d3d_store st, const int
             __syncwarp();
         }
         __syncthreads();
-        // ---- advance: the new Minkowski point (gjk_step_begin after the supports)
+        // ---- advance: the new Minkowski point (gjk_step between its supports and its solve)
         int cls = -1;
         if (state == kLive) {
             const unsigned mt = m.meta[t];

@@ -1,8 +1,10 @@
-// jolt.cuh -- Jolt / van den Bergen GJK on the device, one thread per pair.
+// jolt.cuh -- Jolt / van den Bergen GJK on the device: its sub-algorithms, used
+// by the pools (gjk_pool.cuh) and the mixed form, and the loop of one pair on
+// one thread (the vertex-cached distance).
 //
-// The simplex lives in registers: Y (Minkowski-difference points), P and Q
-// (support points on each collider), four rows each, indexed only by
-// compile-time constants after unrolling.  Sub-algorithms follow
+// The one-thread simplex: Y (Minkowski-difference points) in registers, indexed
+// only by compile-time constants after unrolling, P and Q (support points on
+// each collider) in registers or shared memory, four rows each.  Sub-algorithms follow
 // distance3d gjk/_gjk_jolt.py (cited per function); all thresholds come in
 // through JoltEps so the FP32 phase of the mixed form can scale them.
 #pragma once
@@ -302,7 +304,7 @@ __device__ __forceinline__ void simplex_push(Simplex<T, Rows>& S, V3<T> w, V3<T>
 
 // keep the rows whose bit is set, in order (_gjk_jolt.py:655-664); rows at
 // and above the new count keep their old contents, as in the reference
-template <typename T, bool WITH_PQ, typename Rows>
+template <typename T, typename Rows>
 __device__ __forceinline__ void simplex_compact(Simplex<T, Rows>& S, int set) {
     int m = 0;
 #pragma unroll
@@ -312,7 +314,7 @@ __device__ __forceinline__ void simplex_compact(Simplex<T, Rows>& S, int set) {
             for (int j = 0; j <= i; ++j)
                 if (j == m && j != i) {
                     S.Y[j] = S.Y[i];
-                    if (WITH_PQ) S.R.move(j, i);
+                    S.R.move(j, i);
                 }
             ++m;
         }
@@ -429,15 +431,6 @@ __device__ __forceinline__ void closest_points(const Simplex<T, Rows>& S, const 
 
 enum GjkEnd { GJK_NO_INTERSECTION = 0, GJK_INTERSECTION = 1, GJK_CLIPPED = 3 };
 
-
-// Support evaluated in the loop's own precision (the reference's function).
-struct ExactSupport {
-    template <typename T>
-    static __device__ __forceinline__ V3<T> eval(const Col<T>& c, const d3d_store& s, V3<T> d) {
-        return support(c, s, d);
-    }
-};
-
 // Support points p of collider a along d and q of collider b along -d.  The
 // records are read from the store (L1-resident) inside a two-trip loop, so
 // the support code exists once per kernel and holds no registers across the
@@ -507,20 +500,11 @@ __device__ __forceinline__ void gjk_begin(GjkLoop<T, Rows>& g, V3<T> dir, T vl, 
 }
 
 // One iteration of gjk_distance_jolt's loop (_gjk_jolt.py:200-210) with
-// _distance_loop (:224-288) inlined; returns true once the loop has ended.
-//
-// GAP adds the duality-gap termination of van den Bergen's GJK, which the
-// reference does not have: with v the current closest point and w the new
-// support point along -v, |v| - (|v|^2 - v.w) / |v| <= distance <= |v|.  The
-// loop stops once that bracket is within rel_gap |v| (relative) or within
-// sqrt(abs_gap2) max(1, |w|) (absolute, on the scene's scale).  The FP64
-// drop-in is compiled without it.  A non-null `mesh_cache` (two ints) takes
-// the reference's supports with MeshGraph vertex caching
-// (pair_supports_cached) instead of Sup.
-template <typename T, typename Sup = ExactSupport, bool GAP = false, typename Rows>
-__device__ __forceinline__ bool gjk_step_begin(GjkLoop<T, Rows>& g, const d3d_store& st, int a, int b, T max_d2,
-                                               int max_iter, T rel_gap = T(0), T abs_gap2 = T(0),
-                                               int* mesh_cache = nullptr) {
+// _distance_loop (:224-288) inlined, the supports with MeshGraph vertex caching
+// (pair_supports_cached); returns true once the loop has ended.
+template <typename T, typename Rows>
+__device__ __forceinline__ bool gjk_step(GjkLoop<T, Rows>& g, const d3d_store& st, int a, int b, T tol_sq, T max_d2,
+                                         int max_iter, const JoltEps<T>& E, int* mesh_cache) {
     if (g.it >= max_iter) {
         g.status = D3D_STATUS_MAX_ITER;
         g.state = GJK_NO_INTERSECTION;
@@ -529,10 +513,7 @@ __device__ __forceinline__ bool gjk_step_begin(GjkLoop<T, Rows>& g, const d3d_st
     ++g.it;
     const unsigned together = __activemask();
     V3<T> p, q;
-    if (mesh_cache)
-        pair_supports_cached<T>(st, a, b, g.dir, p, q, mesh_cache);
-    else
-        pair_supports<T, Sup>(st, a, b, g.dir, p, q);
+    pair_supports_cached<T>(st, a, b, g.dir, p, q, mesh_cache);
     // The supports branch by collider type and polytope size; without this
     // the lanes would reach the simplex solve in the groups those branches
     // left and run it once per group.
@@ -543,25 +524,11 @@ __device__ __forceinline__ bool gjk_step_begin(GjkLoop<T, Rows>& g, const d3d_st
         g.state = GJK_CLIPPED;
         return true;
     }
-    if (GAP && g.S.n > 0) {
-        // gap = |v|^2 - v.w >= 0 (up to rounding): |v| - gap / |v| <= distance <= |v|
-        const T gap = g.vl + dd;
-        if (gap <= rel_gap * g.vl || gap * gap <= abs_gap2 * maxf2(T(1), dot(w, w)) * g.vl) {
-            g.dir = -g.dir;  // the state the reference leaves on convergence
-            g.state = GJK_NO_INTERSECTION;
-            return true;
-        }
-    }
     simplex_push(g.S, w, p, q);
-    return false;
-}
-
-// The rest of the iteration, given the result of
-// closest_to_origin(g.S, g.prev, E, nv, nl, set) (`closer`: its return value).
-template <typename T, typename Rows>
-__device__ __forceinline__ bool gjk_step_end(GjkLoop<T, Rows>& g, T tol_sq, const JoltEps<T>& E, bool closer,
-                                             V3<T> nv, T nl, int set) {
-    if (closer) {
+    V3<T> nv = mk(T(0), T(0), T(0));
+    T nl = T(0);
+    int set = 0;
+    if (closest_to_origin(g.S, g.prev, E, nv, nl, set)) {
         g.dir = nv;
         g.vl = nl;
     } else {
@@ -573,7 +540,7 @@ __device__ __forceinline__ bool gjk_step_end(GjkLoop<T, Rows>& g, T tol_sq, cons
         g.state = GJK_INTERSECTION;
         return true;
     }
-    simplex_compact<T, true>(g.S, set);
+    simplex_compact(g.S, set);
     if (le_sq(g.vl, tol_sq) || le_sq(g.vl, E.isect * max_y_len_sq(g.S))) {
         g.vl = T(0);
         g.state = GJK_INTERSECTION;
@@ -586,20 +553,6 @@ __device__ __forceinline__ bool gjk_step_end(GjkLoop<T, Rows>& g, T tol_sq, cons
     }
     g.prev = g.vl;
     return false;
-}
-
-// One iteration: gjk_step_begin, the simplex solve, gjk_step_end (kernels
-// that solve the simplices of a block together call the halves themselves).
-template <typename T, typename Sup = ExactSupport, bool GAP = false, typename Rows>
-__device__ __forceinline__ bool gjk_step(GjkLoop<T, Rows>& g, const d3d_store& st, int a, int b, T tol_sq, T max_d2,
-                                         int max_iter, const JoltEps<T>& E, T rel_gap = T(0), T abs_gap2 = T(0),
-                                         int* mesh_cache = nullptr) {
-    if (gjk_step_begin<T, Sup, GAP>(g, st, a, b, max_d2, max_iter, rel_gap, abs_gap2, mesh_cache)) return true;
-    V3<T> nv = mk(T(0), T(0), T(0));
-    T nl = T(0);
-    int set = 0;
-    const bool closer = closest_to_origin(g.S, g.prev, E, nv, nl, set);
-    return gjk_step_end(g, tol_sq, E, closer, nv, nl, set);
 }
 
 // After the loop: closest points, sanity check, distance
