@@ -959,7 +959,7 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_epa_exact_block(d3d_store s,
             md = key_dist(K[closest]);
             sd = P.normal(closest);
             // supports: a box or hull by its half warp here (first maximum of V . d, a NaN at vertex
-            // 0 wins, later NaNs never do); the other types are posted for warp 0
+            // 0 wins, later NaNs never do); the other types are posted for the block
             const bool up = ln & 16;
             const unsigned half = up ? 0xffff0000u : 0x0000ffffu;
             const int side = up ? 1 : 0;

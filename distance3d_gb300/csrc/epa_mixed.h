@@ -31,7 +31,7 @@ int epa_mixed_launch(const d3d_store& store, const int32_t* i1, const int32_t* i
 // as above.  The FP32 form writes each converged pair's FP32 face normal to
 // mtv and the pair to refine[*n_refine ...] (the caller zeroes the count, the
 // FP64 form takes neither), and a second kernel then computes the pairs' FP64
-// depths along those normals, one pair per thread.
+// depths along those normals.
 bool epa_warp_supported(const d3d_epa_options& o, bool fp64 = false);
 // Warps per block the form launches under tuning t, as tuned or fewer if their
 // polytopes do not fit in one block.

@@ -29,7 +29,7 @@
 // in epa_mixed.cu.  A pair whose polytope fails validation (degenerate face,
 // horizon not one loop, more horizon edges than max_loose_edges) goes to the
 // fallback list.  The converged face is refined along its FP32 normal with
-// FP64 supports in a second pass, one pair per thread (k_epa_refine).
+// FP64 supports in a second pass, the supports listed by type (k_epa_refine).
 //
 // The same search is instantiated with an FP64 polytope and exact FP64
 // supports.  It takes the FP32 search's fallback pairs: the plane tests
@@ -782,6 +782,7 @@ __global__ void __launch_bounds__(32 * WARPS, seg_warps(W) / WARPS) k_epa_segmen
     unsigned long long* __restrict__ n_fallback, int32_t* __restrict__ refine,
     unsigned long long* __restrict__ n_refine, int64_t lo, int64_t hi) {
     using S = Seg<W>;
+    static_assert(kSegChunk >= S::kPairs, "a claim serves every segment that asks");
     constexpr int H = W / 2;        // lanes per collider
     constexpr int kRun = -1000;     // no outcome yet
     extern __shared__ __align__(16) unsigned char smem[];

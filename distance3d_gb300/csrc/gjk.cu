@@ -1,5 +1,6 @@
-// gjk.cu -- the plain FP64 GJK drop-in: batched distance and intersection,
-// one thread per pair.  Compiled with -fmad=false so that the arithmetic is
+// gjk.cu -- the plain FP64 GJK drop-in: batched distance and intersection, a
+// pool of pairs per block (gjk_pool.cuh), and the distance with MeshGraph vertex
+// caching, one thread per pair.  Compiled with -fmad=false so that the arithmetic is
 // the reference's rounding sequence (see d3d_device.cuh); the results are the
 // reference's bit for bit.
 #include "capi_util.h"

@@ -1,6 +1,7 @@
 // gjk_mixed.cu -- mixed-precision GJK distance.
 //
-// Five kernels over the type-sorted pair order:
+// Five kernels, over the pairs in type-sorted order where the batch fills phase
+// A's grid (mixed_sorted), else in input order:
 //
 // A  runs the Jolt loop in FP32 on the FP32 mirror of the store, with
 //    thresholds scaled to single precision, hands each pair's outcome, final
@@ -19,7 +20,7 @@
 //    coordinates; so is a touching pair whose FP64 tetrahedron encloses the
 //    origin.  Every other separated or touching pair is flagged, its FP64 rows
 //    in its record, and a stable compaction (CUB) lists the flagged pairs in
-//    the type-sorted order.
+//    the order of the slots.
 // B  continues the reference's loop (_gjk_jolt.py:224-288) in FP64 for the
 //    listed pairs, a pool of pairs per block: the first round solves the
 //    handed rows, later rounds add a support pair along -v, until the duality
@@ -466,7 +467,7 @@ __global__ void __launch_bounds__(BLOCK) k_gjk_mixed_r(d3d_store s, const int32_
     }
 }
 
-// B over R's run list, in the type-sorted order: a pool of S pairs per block
+// B over R's run list, in the order of the slots: a pool of S pairs per block
 // in shared memory, in rounds as the plain FP64 GJK runs them (gjk_pool.cuh,
 // whose pool it uses).  Each round lists the pairs' supports by collider type
 // (a hull is searched by the whole warp) and, after the new Minkowski points,
@@ -766,7 +767,7 @@ __global__ void __launch_bounds__(S, 3) k_gjk_mixed_b(d3d_store st, const int32_
 __global__ void __launch_bounds__(128) k_gjk_mixed_end(d3d_gjk_options opt, DistanceOut o, Lists lists) {
     const int64_t n = (int64_t)lists.ctr[kNumEnd];
     const JoltEps<double> E = reference_eps<double>();
-    const int64_t lanes = spread_lanes(n, 128), warps = (int64_t)gridDim.x * 4;  // as in B
+    const int64_t lanes = spread_lanes(n, 128), warps = (int64_t)gridDim.x * 4;  // few pairs: spread
     const int ln = threadIdx.x & 31;
     if (ln >= lanes) return;
     for (int64_t k = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * lanes + ln; k < n; k += warps * lanes) {

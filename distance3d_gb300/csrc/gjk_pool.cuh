@@ -1,6 +1,6 @@
 // gjk_pool.cuh -- the FP64 GJK over a pool of pairs per block.
 //
-// What bounds it: the FP64 pipe, which takes one warp instruction per 19
+// What bounds it: the FP64 pipe, which takes one warp instruction per 16
 // cycles of an SM (64 from a single warp) however few lanes are active, and
 // the length of a pair's chain of iterations (19 on average, ~75 at most).
 // With one lane per pair the lanes of a warp sit in different support
@@ -242,9 +242,10 @@ __device__ __forceinline__ void lane_support(M& m, const d3d_store& st, int e) {
     m.put_support(s, side, support(c, st, d));
 }
 
-// The rest of gjk_step after its solve (distance) or the rest of the intersection test's iteration
-// (gjk_intersection_jolt, _gjk_jolt.py:29-135), for slot s and the result of its solve; ysq(r) is |Y|^2 of place r.  Returns
-// the intersection form's outcome, -1 while it runs.
+// The rest of gjk_step after its solve (distance) or of the intersection test's
+// iteration (gjk_intersection_jolt, _gjk_jolt.py:29-135), for slot s and the
+// result of its solve; ysq(r) is |Y|^2 of place r.  Returns the intersection
+// form's outcome, -1 while it runs.
 template <int S, int PQ, typename Ysq>
 __device__ __forceinline__ int finish_step(Mem<S, PQ>& m, int s, bool closer, d3 nv, double nl, int set, double tol_sq,
                                            int max_iter, const JoltEps<double>& E, Ysq ysq) {

@@ -39,7 +39,7 @@ struct WarpChunk {
 
 // Lanes with `need` set receive consecutive slots (-1 for the others), taken
 // from the warp's chunk; when the chunk runs out the warp claims the next
-// `chunk` (>= 32) slots of *cursor.  A warp's lanes then hold pairs from at
+// `chunk` slots of *cursor (at least as many as lanes can ask at once).  A warp's lanes then hold pairs from at
 // most two chunks of the order at a time, instead of from anywhere in the
 // span all resident lanes of the GPU have fetched, which keeps the lanes of
 // a warp on pairs of the same collider types in a type-sorted order.  Once
