@@ -107,17 +107,16 @@ __global__ void __launch_bounds__(BLOCK, phase_a_min_blocks<BLOCK>()) k_gjk_mixe
     int64_t pid = 0;
     int a = 0, b = 0;
     const long long lanes = spread_lanes(n, BLOCK);
-    bool have = false, bad = false;
-    int part = lane_part((int)(threadIdx.x & 31) < lanes);
+    bool have = false, bad = false, exhausted = false;
+    bool spare = (int)(threadIdx.x & 31) >= lanes;  // sits out the first round (persist.cuh)
     WarpChunk chunk;
     while (true) {
         __syncwarp();
-        part = next_part(part, lists.ctr + kCurA, n);
-        const bool want = !have && part == 0;
+        const bool want = !have && !exhausted && !spare;
         const long long slot = fetch_slot_chunked(lists.ctr + kCurA, want, chunk, kAll, kChunk, 0);
         if (want) {
             if (slot >= n) {
-                part = kOut;
+                exhausted = true;
             } else {
                 pid = order ? order[slot] : slot;
                 a = i1[pid];
@@ -126,6 +125,10 @@ __global__ void __launch_bounds__(BLOCK, phase_a_min_blocks<BLOCK>()) k_gjk_mixe
                 pa_begin(L);
                 have = true;
             }
+        }
+        if (spare) {
+            exhausted = slots_claimed(lists.ctr + kCurA, n);
+            spare = false;
         }
         if (!__any_sync(kAll, have)) break;
         int o = pa_step<MESH, true>(L, have && !bad, s, a, b, tol_sq, max_d2, max_iter);
@@ -478,7 +481,8 @@ __global__ void __launch_bounds__(BLOCK) k_gjk_mixed_r(d3d_store s, const int32_
 // FP64 instruction: 87,819 scene pairs 385 -> 361 us, 300,032 robot pairs
 // 356 -> 299 us, 20,011 pairs of ten types 222 -> 187 us, 3,000 pairs 120 ->
 // 107 us, 1M pairs 727 -> 720 us.
-constexpr int kReplay = 3;  // state beside pool::kFree, kLive
+// states beside pool::kFree and kLive (the loop has no kEnding)
+constexpr int kReplay = pool::kEnding, kSpare = pool::kSpare;
 
 template <int S>
 __device__ __forceinline__ void b_finish(const pool::Mem<S, 4>& m, int s, unsigned perm, int n, d3 dir, double vl,
@@ -534,9 +538,9 @@ __global__ void __launch_bounds__(S, 3) k_gjk_mixed_b(d3d_store st, const int32_
     const double tol_sq = opt.tolerance * opt.tolerance;
     const long long share = (n + gridDim.x - 1) / gridDim.x;
     const long long split = share < S ? 0 : n;
-    int part = lane_part(t < share);
+    bool exhausted = share == 0;
     WarpChunk chunk;
-    m.meta[t] = 0;
+    m.meta[t] = !exhausted && t >= share ? pool::pack_meta(0, 0, 0, kSpare) : 0;
     if (t < kBins) m.cnt[0][t] = m.cnt[1][t] = 0;
     if (t < 4) m.scnt[0][t] = m.scnt[1][t] = m.next[t >> 1][t & 1] = 0;
     int type[2] = {0, 0};
@@ -544,12 +548,11 @@ __global__ void __launch_bounds__(S, 3) k_gjk_mixed_b(d3d_store st, const int32_
     for (int par = 0;; par ^= 1) {
         // ---- free slots take new pairs
         int state = pool::meta_state(m.meta[t]);
-        part = next_part(part, lists.ctr + kCurB, n);
-        const bool want = state == pool::kFree && part == 0;
+        const bool want = state == pool::kFree && !exhausted;
         const long long slot = fetch_slot_chunked(lists.ctr + kCurB, want, chunk, kAll, kChunk, split);
         if (want) {
             if (slot >= n) {
-                part = kOut;
+                exhausted = true;
             } else {
                 const int pid = lists.run[slot];
                 const EndRecord& rec = lists.records[pid];
@@ -594,7 +597,7 @@ __global__ void __launch_bounds__(S, 3) k_gjk_mixed_b(d3d_store st, const int32_
             if (ln == leader && bin >= 0) base = atomicAdd(&m.cnt[par][bin], __popc(same));
             pos[k] = __shfl_sync(kAll, base, leader) + __popc(same & ((1u << ln) - 1u));
         }
-        if (!__syncthreads_or(state != pool::kFree || part == 0)) break;
+        if (!__syncthreads_or(state != pool::kFree || !exhausted)) break;
         const Chunks ch = chunks_of(m.cnt[par], kBins, (ln >> 1) == D3D_HULL ? pool::kHullChunk : 32);
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
@@ -665,6 +668,9 @@ __global__ void __launch_bounds__(S, 3) k_gjk_mixed_b(d3d_store st, const int32_
                 lists.fallback[atomicAdd(lists.ctr + kNumFallback, 1ull)] = m.pid[t];
                 m.meta[t] = 0;
             }
+        } else if (state == kSpare) {
+            exhausted = slots_claimed(lists.ctr + kCurB, n);
+            m.meta[t] = 0;
         }
         __syncwarp();
         {

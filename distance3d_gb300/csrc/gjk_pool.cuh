@@ -50,7 +50,7 @@ constexpr int kTetraChunk = 16;  // tetrahedra per chunk: ~27 of their faces see
 constexpr int kEndMin = 32;      // finished pairs that make an end chunk worth running
 constexpr int kFetch = 32;       // pairs a warp claims from the order at a time
 
-enum { kFree = 0, kLive = 1, kEnding = 2 };
+enum { kFree = 0, kLive = 1, kEnding = 2, kSpare = 3 };  // kSpare: sits out the first round (persist.cuh)
 
 // a pair's state word
 __device__ __forceinline__ unsigned pack_meta(unsigned perm, int n, int fresh, int state, int gstate = 0,
@@ -665,11 +665,11 @@ __global__ void __launch_bounds__(S, 512 / S) k_gjk_pool(d3d_store st, const int
     // a batch that does not fill every block is spread evenly over them
     const long long share = (n + gridDim.x - 1) / gridDim.x;
     const long long split = share < S ? 0 : n;
-    int part = kDistance ? lane_part(t < share) : (t < share ? 0 : kOut);
+    bool exhausted = kDistance ? share == 0 : t >= share;
     WarpChunk chunk;
     __shared__ unsigned dealt;
     if (!kDistance && t == 0) dealt = 0u;
-    m.meta[t] = 0;
+    m.meta[t] = !exhausted && t >= share ? pack_meta(0, 0, 0, kSpare) : 0;
     if (t < kBins) m.cnt[0][t] = m.cnt[1][t] = 0;
     if (t < 4) m.scnt[0][t] = m.scnt[1][t] = m.next[t >> 1][t & 1] = 0;
     int type0 = 0, type1 = 0;
@@ -677,13 +677,12 @@ __global__ void __launch_bounds__(S, 512 / S) k_gjk_pool(d3d_store st, const int
     for (int par = 0;; par ^= 1) {
         // ---- free slots take new pairs
         int state = meta_state(m.meta[t]);
-        if (kDistance) part = next_part(part, cursor, n);
-        const bool want = state == kFree && part == 0;
+        const bool want = state == kFree && !exhausted;
         const long long slot = kDistance ? fetch_slot_chunked(cursor, want, chunk, kAll, kFetch, split)
                                          : (long long)dealt_slot(&dealt, want, share < S ? 0 : 5);
         if (want) {
             if (slot >= n) {
-                part = kOut;
+                exhausted = true;
             } else {
                 const int pid = order ? order[slot] : (int)slot;
                 const int a = i1[pid], b = i2[pid];
@@ -724,7 +723,7 @@ __global__ void __launch_bounds__(S, 512 / S) k_gjk_pool(d3d_store st, const int
             if (ln == leader && bin >= 0) base = atomicAdd(&m.cnt[par][bin], __popc(same));
             pos[k] = __shfl_sync(kAll, base, leader) + __popc(same & ((1u << ln) - 1u));
         }
-        if (!__syncthreads_or(state != kFree || part == 0)) break;
+        if (!__syncthreads_or(state != kFree || !exhausted)) break;
         // bin ln of the list: its first task and first chunk; the finished pairs wait until they
         // fill a warp, or no pair is left to iterate
         const int size = (ln >> 1) == D3D_HULL ? kHullChunk : 32;
@@ -814,6 +813,9 @@ __global__ void __launch_bounds__(S, 512 / S) k_gjk_pool(d3d_store st, const int
                 m.meta[t] = pack_meta(perm, rows + 1, 0, kLive);
                 cls = 3 - rows;  // 0: tetrahedron .. 3: point
             }
+        } else if (kDistance && state == kSpare) {
+            exhausted = slots_claimed(cursor, n);
+            m.meta[t] = 0;
         }
         {
             unsigned mine = 0;

@@ -36,7 +36,7 @@ constexpr int kInit = 5;  // phase of a pair whose portal is not begun
 constexpr int kPhases = 6;
 
 using PortalT = mpr::Portal<double, kSlots, true>;
-enum { kFree = 0, kLive = 1, kEnding = 2 };
+enum { kFree = 0, kLive = 1, kEnding = 2, kSpare = 3 };  // kSpare: sits out the first round (persist.cuh)
 
 struct Mem {
     double rows[PortalT::kWords * kSlots];
@@ -114,9 +114,9 @@ __global__ void __launch_bounds__(kSlots, 2) k_mpr(d3d_store st, const int32_t* 
     // a batch that does not fill every block is spread evenly over them
     const long long share = (n + gridDim.x - 1) / gridDim.x;
     const long long split = share < kSlots ? 0 : n;
-    int part = lane_part(t < share);
+    bool exhausted = share == 0;
     WarpChunk chunk;
-    m.meta[t] = 0;
+    m.meta[t] = !exhausted && t >= share ? kSpare : kFree;
     if (t < kBins) m.cnt[0][t] = m.cnt[1][t] = 0;
     if (t < kPhases) m.scnt[0][t] = m.scnt[1][t] = 0;
     if (t < 2) m.next[0][t] = m.next[1][t] = 0;
@@ -125,12 +125,11 @@ __global__ void __launch_bounds__(kSlots, 2) k_mpr(d3d_store st, const int32_t* 
     for (int par = 0;; par ^= 1) {
         // ---- free slots take new pairs
         int meta = m.meta[t];
-        part = next_part(part, cursor, n);
-        const bool want = (meta & 3) == kFree && part == 0;
+        const bool want = (meta & 3) == kFree && !exhausted;
         const long long slot = fetch_slot_chunked(cursor, want, chunk, kAll, 32, split);
         if (want) {
             if (slot >= n) {
-                part = kOut;
+                exhausted = true;
             } else {
                 const int pid = order ? order[slot] : (int)slot;
                 const int c[2] = {i1[pid], i2[pid]};
@@ -166,7 +165,7 @@ __global__ void __launch_bounds__(kSlots, 2) k_mpr(d3d_store st, const int32_t* 
             if (ln == leader && bin[k] >= 0) base = atomicAdd(&m.cnt[par][bin[k]], __popc(same));
             pos[k] = __shfl_sync(kAll, base, leader) + __popc(same & ((1u << ln) - 1u));
         }
-        const int running = __syncthreads_or((state != kFree || part == 0 ? 1 : 0) | (state == kLive ? 2 : 0));
+        const int running = __syncthreads_or((state != kFree || !exhausted ? 1 : 0) | (state == kLive ? 2 : 0));
         if (!running) break;
         // the finished pairs wait until they fill a warp, or no pair is left to iterate
         const bool ends = m.cnt[par][kEndBin] >= 32 || !(running & 2);
@@ -213,6 +212,10 @@ __global__ void __launch_bounds__(kSlots, 2) k_mpr(d3d_store st, const int32_t* 
             }
             const int p = __shfl_sync(kAll, base, cls >= 0 ? cls : 0) + __popc(mine & ((1u << ln) - 1u));
             if (cls >= 0) m.step[cls * kSlots + p] = (unsigned short)t;
+        }
+        if (state == kSpare) {
+            exhausted = slots_claimed(cursor, n);
+            m.meta[t] = kFree;
         }
         // the other parity's counters, free since the last round
         if (t < kBins) m.cnt[par ^ 1][t] = 0;

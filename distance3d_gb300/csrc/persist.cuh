@@ -84,24 +84,17 @@ __device__ __forceinline__ long long fetch_slot_chunked(unsigned long long* curs
 // is right while all its blocks run at once.  Where other batches hold part of
 // the GPU, the blocks that do run would go through share after share, and the
 // batches beside this one would wait for its blocks: so a lane beyond the share
-// sits out kSpreadRounds rounds only and then takes what is left, and the
-// blocks that start later find nothing and end.  One round covers the start of
-// a grid that has the GPU to itself: 1, 3 and 7 measured the same for 1,000 to
-// 65,536 pairs, 0 (as dense as the lanes allow) 895 -> 1,950 us for 4,096 FP64
-// pairs.  Batches of 4,096 six-type pairs on 16 streams, M pairs/s, without ->
-// with 7, 3, 1 rounds: FP64 GJK 6.7 -> 19.5, 21.8, 22.3; mixed GJK 44.7 ->
-// 42.7, 46.6, 48.1; MPR 28 -> 39, 47, 46.
-constexpr int kSpreadRounds = 1;
+// sits out one round only and then takes what is left, and the blocks that
+// start later find nothing and end.  One round covers the start of a grid that
+// has the GPU to itself: 1, 3 and 7 measured the same for 1,000 to 65,536 pairs,
+// 0 (as dense as the lanes allow) 895 -> 1,950 us for 4,096 FP64 pairs.  Batches
+// of 4,096 six-type pairs on 16 streams, M pairs/s, without -> with 7, 3, 1
+// rounds: FP64 GJK 6.7 -> 19.5, 21.8, 22.3; mixed GJK 44.7 -> 42.7, 46.6, 48.1;
+// MPR 28 -> 39, 47, 46.
 
-// A lane's part in the fetches: 0 takes pairs, kOut is out of the batch, and a
-// positive count sits out.
-constexpr int kOut = -1;
-__device__ __forceinline__ int lane_part(bool in_share) { return in_share ? 0 : kSpreadRounds + 1; }
-// at the start of a round, for a batch of n slots
-__device__ __forceinline__ int next_part(int part, const unsigned long long* cursor, long long n) {
-    if (part > 0 && --part == 0 && (long long)*reinterpret_cast<const volatile unsigned long long*>(cursor) >= n)
-        part = kOut;
-    return part;
+// Whether every slot below n is claimed.
+__device__ __forceinline__ bool slots_claimed(const unsigned long long* cursor, long long n) {
+    return (long long)*reinterpret_cast<const volatile unsigned long long*>(cursor) >= n;
 }
 
 // Lanes with `take` set append `value` to list[*count ...], one atomic per

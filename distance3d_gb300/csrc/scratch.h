@@ -37,10 +37,11 @@ private:
 bool shared_gpu();
 
 // A server of more slots than this, or the tuner for as many batches, launches
-// for a shared GPU.  A batch of 4,096 pairs alone on the whole GPU takes 0.57
-// ms instead of 0.77, but 16 slots of them run one after the other.  Peak M
-// pairs/s of 2,000-pair requests with / without: 16 slots 51.3 / 31.7 (FP64
-// 10.4 / 8.8), 8 slots 32.8 / 28.2, 4 slots 18.0 / 21.3 (FP64 5.3 / 4.8).
+// for a shared GPU.  A batch of 4,096 pairs alone on the whole GPU takes 0.56
+// ms instead of 0.76, but its unsorted FP32 phase and whole-warp EPA cost the
+// batches beside it more.  Peak M pairs/s of 2,000-pair requests with /
+// without: 16 slots 51.0 / 36.3 (FP64 10.3 / 9.7), 8 slots 32.7 / 30.0 (8.4 /
+// 7.7), 4 slots 18.1 / 19.6 (5.3 / 4.8; one request 2.19 / 1.66 ms).
 constexpr size_t kAloneBatches = 4;
 
 // Work items to size a small batch's launch by: `alone` or, beside other batches, `dense`.
