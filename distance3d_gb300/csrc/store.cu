@@ -465,7 +465,10 @@ extern "C" int d3d_store_pack(const d3d_store* store, const int32_t* types, cons
     rc = d3d::scratch_alloc(&block, sizeof(int), st);
     if (rc) return rc;
     int* const bad = static_cast<int*>(block);
-    cudaMemsetAsync(bad, 0, sizeof(int), st);
+    if (cudaMemsetAsync(bad, 0, sizeof(int), st) != cudaSuccess) {
+        d3d::scratch_free(block, st);
+        return d3d::check_launch("d3d_store_pack: flag");
+    }
     if (n_hull_vertices > 0) k_hull_to_f32<<<d3d::grid_for(n_hull_vertices, 256), 256, 0, st>>>(*store, n_hull_vertices);
     if (n > 0)
         k_pack<<<d3d::grid_for(n, 128), 128, 0, st>>>(*store, types, poses, params, hull_offset, hull_count, n, bad);
