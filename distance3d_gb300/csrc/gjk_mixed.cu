@@ -108,11 +108,12 @@ __global__ void __launch_bounds__(BLOCK, phase_a_min_blocks<BLOCK>()) k_gjk_mixe
     int a = 0, b = 0;
     const long long lanes = spread_lanes(n, BLOCK);
     bool have = false, bad = false, exhausted = false;
-    bool spare = (int)(threadIdx.x & 31) >= lanes;  // sits out the first round (persist.cuh)
+    // rounds the lane sits out (persist.cuh)
+    int spare = (int)(threadIdx.x & 31) >= lanes && lanes ? spare_rounds(threadIdx.x & 31, lanes) : 0;
     WarpChunk chunk;
     while (true) {
         __syncwarp();
-        const bool want = !have && !exhausted && !spare;
+        const bool want = !have && !exhausted && spare == 0;
         const long long slot = fetch_slot_chunked(lists.ctr + kCurA, want, chunk, kAll, kChunk, 0);
         if (want) {
             if (slot >= n) {
@@ -126,10 +127,6 @@ __global__ void __launch_bounds__(BLOCK, phase_a_min_blocks<BLOCK>()) k_gjk_mixe
                 have = true;
             }
         }
-        if (spare) {
-            exhausted = slots_claimed(lists.ctr + kCurA, n);
-            spare = false;
-        }
         if (!__any_sync(kAll, have)) break;
         int o = pa_step<MESH, true>(L, have && !bad, s, a, b, tol_sq, max_d2, max_iter);
         if (have && bad) o = PA_BAD_INDEX;
@@ -138,6 +135,10 @@ __global__ void __launch_bounds__(BLOCK, phase_a_min_blocks<BLOCK>()) k_gjk_mixe
             hand[pid] = pa_handoff(L, o);
             if (bad) store_bad_index(out, pid);
             have = false;
+        }
+        if (spare) {
+            exhausted = slots_claimed(lists.ctr + kCurA, n);
+            spare = exhausted ? 0 : spare - 1;
         }
         __syncwarp();
         append_lanes(kAll, lists.fallback, lists.ctr + kNumFallback, done && (o == PA_CLIPPED || o == PA_FAILED),
@@ -541,6 +542,7 @@ __global__ void __launch_bounds__(S, 3) k_gjk_mixed_b(d3d_store st, const int32_
     bool exhausted = share == 0;
     WarpChunk chunk;
     m.meta[t] = !exhausted && t >= share ? pool::pack_meta(0, 0, 0, kSpare) : 0;
+    if (!exhausted && t >= share) m.it[t] = spare_rounds(t, share);
     if (t < kBins) m.cnt[0][t] = m.cnt[1][t] = 0;
     if (t < 4) m.scnt[0][t] = m.scnt[1][t] = m.next[t >> 1][t & 1] = 0;
     int type[2] = {0, 0};
@@ -597,7 +599,7 @@ __global__ void __launch_bounds__(S, 3) k_gjk_mixed_b(d3d_store st, const int32_
             if (ln == leader && bin >= 0) base = atomicAdd(&m.cnt[par][bin], __popc(same));
             pos[k] = __shfl_sync(kAll, base, leader) + __popc(same & ((1u << ln) - 1u));
         }
-        if (!__syncthreads_or(state != pool::kFree || !exhausted)) break;
+        if (!__syncthreads_or(state == pool::kFree ? !exhausted : state != kSpare)) break;
         const Chunks ch = chunks_of(m.cnt[par], kBins, (ln >> 1) == D3D_HULL ? pool::kHullChunk : 32);
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
@@ -670,7 +672,7 @@ __global__ void __launch_bounds__(S, 3) k_gjk_mixed_b(d3d_store st, const int32_
             }
         } else if (state == kSpare) {
             exhausted = slots_claimed(lists.ctr + kCurB, n);
-            m.meta[t] = 0;
+            if (exhausted || --m.it[t] == 0) m.meta[t] = 0;
         }
         __syncwarp();
         {

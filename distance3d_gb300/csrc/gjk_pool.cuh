@@ -50,7 +50,7 @@ constexpr int kTetraChunk = 16;  // tetrahedra per chunk: ~27 of their faces see
 constexpr int kEndMin = 32;      // finished pairs that make an end chunk worth running
 constexpr int kFetch = 32;       // pairs a warp claims from the order at a time
 
-enum { kFree = 0, kLive = 1, kEnding = 2, kSpare = 3 };  // kSpare: sits out the first round (persist.cuh)
+enum { kFree = 0, kLive = 1, kEnding = 2, kSpare = 3 };  // kSpare: beyond the share (persist.cuh)
 
 // a pair's state word
 __device__ __forceinline__ unsigned pack_meta(unsigned perm, int n, int fresh, int state, int gstate = 0,
@@ -670,6 +670,7 @@ __global__ void __launch_bounds__(S, 512 / S) k_gjk_pool(d3d_store st, const int
     __shared__ unsigned dealt;
     if (!kDistance && t == 0) dealt = 0u;
     m.meta[t] = !exhausted && t >= share ? pack_meta(0, 0, 0, kSpare) : 0;
+    if (!exhausted && t >= share) m.it[t] = spare_rounds(t, share);
     if (t < kBins) m.cnt[0][t] = m.cnt[1][t] = 0;
     if (t < 4) m.scnt[0][t] = m.scnt[1][t] = m.next[t >> 1][t & 1] = 0;
     int type0 = 0, type1 = 0;
@@ -723,7 +724,7 @@ __global__ void __launch_bounds__(S, 512 / S) k_gjk_pool(d3d_store st, const int
             if (ln == leader && bin >= 0) base = atomicAdd(&m.cnt[par][bin], __popc(same));
             pos[k] = __shfl_sync(kAll, base, leader) + __popc(same & ((1u << ln) - 1u));
         }
-        if (!__syncthreads_or(state != kFree || !exhausted)) break;
+        if (!__syncthreads_or(state == kFree ? !exhausted : state != kSpare)) break;
         // bin ln of the list: its first task and first chunk; the finished pairs wait until they
         // fill a warp, or no pair is left to iterate
         const int size = (ln >> 1) == D3D_HULL ? kHullChunk : 32;
@@ -815,7 +816,7 @@ __global__ void __launch_bounds__(S, 512 / S) k_gjk_pool(d3d_store st, const int
             }
         } else if (kDistance && state == kSpare) {
             exhausted = slots_claimed(cursor, n);
-            m.meta[t] = 0;
+            if (exhausted || --m.it[t] == 0) m.meta[t] = 0;
         }
         {
             unsigned mine = 0;

@@ -36,7 +36,7 @@ constexpr int kInit = 5;  // phase of a pair whose portal is not begun
 constexpr int kPhases = 6;
 
 using PortalT = mpr::Portal<double, kSlots, true>;
-enum { kFree = 0, kLive = 1, kEnding = 2, kSpare = 3 };  // kSpare: sits out the first round (persist.cuh)
+enum { kFree = 0, kLive = 1, kEnding = 2, kSpare = 3 };  // kSpare: beyond the share (persist.cuh)
 
 struct Mem {
     double rows[PortalT::kWords * kSlots];
@@ -117,6 +117,7 @@ __global__ void __launch_bounds__(kSlots, 2) k_mpr(d3d_store st, const int32_t* 
     bool exhausted = share == 0;
     WarpChunk chunk;
     m.meta[t] = !exhausted && t >= share ? kSpare : kFree;
+    if (!exhausted && t >= share) m.it[t] = spare_rounds(t, share);
     if (t < kBins) m.cnt[0][t] = m.cnt[1][t] = 0;
     if (t < kPhases) m.scnt[0][t] = m.scnt[1][t] = 0;
     if (t < 2) m.next[0][t] = m.next[1][t] = 0;
@@ -165,7 +166,7 @@ __global__ void __launch_bounds__(kSlots, 2) k_mpr(d3d_store st, const int32_t* 
             if (ln == leader && bin[k] >= 0) base = atomicAdd(&m.cnt[par][bin[k]], __popc(same));
             pos[k] = __shfl_sync(kAll, base, leader) + __popc(same & ((1u << ln) - 1u));
         }
-        const int running = __syncthreads_or((state != kFree || !exhausted ? 1 : 0) | (state == kLive ? 2 : 0));
+        const int running = __syncthreads_or(((state == kFree ? !exhausted : state != kSpare) ? 1 : 0) | (state == kLive ? 2 : 0));
         if (!running) break;
         // the finished pairs wait until they fill a warp, or no pair is left to iterate
         const bool ends = m.cnt[par][kEndBin] >= 32 || !(running & 2);
@@ -215,7 +216,7 @@ __global__ void __launch_bounds__(kSlots, 2) k_mpr(d3d_store st, const int32_t* 
         }
         if (state == kSpare) {
             exhausted = slots_claimed(cursor, n);
-            m.meta[t] = kFree;
+            if (exhausted || --m.it[t] == 0) m.meta[t] = kFree;
         }
         // the other parity's counters, free since the last round
         if (t < kBins) m.cnt[par ^ 1][t] = 0;

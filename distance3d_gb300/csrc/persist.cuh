@@ -83,14 +83,23 @@ __device__ __forceinline__ long long fetch_slot_chunked(unsigned long long* curs
 // warp) takes its share of the slots and leaves its other lanes empty.  That
 // is right while all its blocks run at once.  Where other batches hold part of
 // the GPU, the blocks that do run would go through share after share, and the
-// batches beside this one would wait for its blocks: so a lane beyond the share
-// sits out one round only and then takes what is left, and the blocks that
-// start later find nothing and end.  One round covers the start of a grid that
-// has the GPU to itself: 1, 3 and 7 measured the same for 1,000 to 65,536 pairs,
-// 0 (as dense as the lanes allow) 895 -> 1,950 us for 4,096 FP64 pairs.  Batches
-// of 4,096 six-type pairs on 16 streams, M pairs/s, without -> with 7, 3, 1
-// rounds: FP64 GJK 6.7 -> 19.5, 21.8, 22.3; mixed GJK 44.7 -> 42.7, 46.6, 48.1;
-// MPR 28 -> 39, 47, 46.
+// batches beside this one would wait for its blocks: so a block's share doubles
+// every round while the cursor is not through, and the blocks that start later
+// find less, or nothing and end.  A batch alone is claimed within its first
+// round and takes the time it takes without this, to within 0.5 % (without any
+// share, as dense as the lanes allow, 895 -> 1,950 us for 4,096 FP64 pairs).
+// Batches of 4,096 six-type pairs on 2 / 4 / 8 / 16 streams, M pairs/s:
+//   FP64 GJK   kept to the share 6.4 / 6.6 / 6.7 / 6.7, all lanes from the
+//              second round on 5.6 / 8.5 / 14.0 / 22.5, doubling 6.9 / 9.3 / 14.1 / 20.9
+//   mixed GJK  23.5 / 36.3 / 43.5 / 44.7, 22.9 / 31.4 / 48.9 / 48.1, 23.4 / 36.9 / 48.3 / 47.7
+//   FP64 MPR   23.3 / 28.0 / 28.4 / 28.3, 19.6 / 31.3 / 40 / 45, 24.1 / 34.8 / 38 / 41
+
+// Rounds that lane t >= share sits out: the share doubles every round.
+__device__ __forceinline__ int spare_rounds(int t, long long share) {
+    int w = 1;
+    while (w < 9 && (share << w) <= t) ++w;
+    return w;
+}
 
 // Whether every slot below n is claimed.
 __device__ __forceinline__ bool slots_claimed(const unsigned long long* cursor, long long n) {

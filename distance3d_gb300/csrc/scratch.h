@@ -40,8 +40,8 @@ bool shared_gpu();
 // for a shared GPU.  A batch of 4,096 pairs alone on the whole GPU takes 0.56
 // ms instead of 0.76, but its unsorted FP32 phase and whole-warp EPA cost the
 // batches beside it more.  Peak M pairs/s of 2,000-pair requests with /
-// without: 16 slots 51.0 / 36.3 (FP64 10.3 / 9.7), 8 slots 32.7 / 30.0 (8.4 /
-// 7.7), 4 slots 18.1 / 19.6 (5.3 / 4.8; one request 2.19 / 1.66 ms).
+// without: 16 slots 50.8 / 31.9 (FP64 10.1 / 8.3), 8 slots 32.7 / 28.0 (8.2 /
+// 7.7), 4 slots 18.1 / 21.5 (5.3 / 5.1; one request 2.19 / 1.66 ms).
 constexpr size_t kAloneBatches = 4;
 
 // Work items to size a small batch's launch by: `alone` or, beside other batches, `dense`.
