@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(S, 512 / S) k_gjk_pool(d3d_store st, const int
     const long long share = (n + gridDim.x - 1) / gridDim.x;
     const long long split = share < S ? 0 : n;
     bool exhausted = kDistance ? share == 0 : t >= share;
-    WarpChunk chunk;
+    WarpChunk32 chunk;
     __shared__ unsigned dealt;
     if (!kDistance && t == 0) dealt = 0u;
     m.meta[t] = !exhausted && t >= share ? pack_meta(0, 0, 0, kSpare) : 0;

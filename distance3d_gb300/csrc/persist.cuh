@@ -33,9 +33,12 @@ __device__ __forceinline__ long long fetch_slot(unsigned long long* cursor, bool
 
 // A warp's share of the global order: the slots [next, end) it has claimed
 // and not yet handed to a lane.  Every lane holds the same copy.
-struct WarpChunk {
-    long long next = 0, end = 0;
+template <typename I>
+struct WarpChunkOf {
+    I next = 0, end = 0;
 };
+using WarpChunk = WarpChunkOf<long long>;
+using WarpChunk32 = WarpChunkOf<unsigned>;  // orders below 2^31
 
 // Lanes with `need` set receive consecutive slots (-1 for the others), taken
 // from the warp's chunk; when the chunk runs out the warp claims the next
@@ -48,7 +51,8 @@ struct WarpChunk {
 // slot waits in the chunk of a busy warp at the end of the order.
 // Every lane of `live` must call it together (converged), so that the
 // lanes' copies of `w` stay equal.
-__device__ __forceinline__ long long fetch_slot_chunked(unsigned long long* cursor, bool need, WarpChunk& w,
+template <typename I>
+__device__ __forceinline__ long long fetch_slot_chunked(unsigned long long* cursor, bool need, WarpChunkOf<I>& w,
                                                         unsigned live, int chunk, long long split) {
     const unsigned want = __ballot_sync(live, need);
     if (!want) return -1;
@@ -73,8 +77,8 @@ __device__ __forceinline__ long long fetch_slot_chunked(unsigned long long* curs
         base = __shfl_sync(live, base, leader);
         size = __shfl_sync(live, size, leader);
         slot = rank < avail ? w.next + rank : (long long)base + (rank - avail);
-        w.next = (long long)base + (cnt - avail);
-        w.end = (long long)base + size;
+        w.next = (I)((long long)base + (cnt - avail));
+        w.end = (I)((long long)base + size);
     }
     return need ? slot : -1;
 }
